@@ -38,7 +38,9 @@ def reference_dir() -> Path:
     """The reference checkout: $DR_REFERENCE, else a directory named `reference` beside
     the repository (the layout oracle/Makefile assumes too)."""
     env = os.environ.get("DR_REFERENCE")
-    return Path(env) if env else ORACLE_DIR.parents[1] / "reference"
+    d = Path(env) if env else ORACLE_DIR.parents[1] / "reference"
+    # an empty directory holds nothing to build from: it counts as absent
+    return d if not d.is_dir() or any(d.iterdir()) else d / "src"
 
 
 def build(ref: bool = True) -> None:
