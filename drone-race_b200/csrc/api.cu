@@ -846,7 +846,7 @@ int buildMppiBatch(dr_mppi* const* hs, int n, cudaStream_t stream, bool ownStrea
     ver.insert(ver.end(), verOld.begin(), verOld.end());
     for (int i = 0; i < n; i++)
     {
-        b->rollSmem = std::max(b->rollSmem, b->envKind ? gateRolloutSmem(b->nth, hs[i]->T, hs[i]->M, b->spl) : mppiRolloutSmem(b->nth, hs[i]->T, hs[i]->M, b->spl));
+        b->rollSmem = std::max(b->rollSmem, b->envKind ? gateRolloutSmem(b->nth, hs[i]->T, hs[i]->M, b->spl) : mppiRolloutSmem(b->nopp, b->nth, hs[i]->T, hs[i]->M, b->spl));
         b->verSmem = std::max(b->verSmem, b->envKind ? gateVerifySmem(b->nth, hs[i]->T) : mppiVerifySmem(b->nth, hs[i]->T));
     }
     b->proSmem = ((size_t)maxNbpT * 2 + (size_t)maxM * 2) * 4;

@@ -61,7 +61,7 @@ constexpr int VERIFY_TILE = DR_VERIFY_TILE;
 
 bool mppiSupported(int nopp, int nth);
 int rolloutSamplesPerBlock(int nth);
-size_t mppiRolloutSmem(int nth, int T, int M, bool spl);
+size_t mppiRolloutSmem(int nopp, int nth, int T, int M, bool spl);
 size_t mppiVerifySmem(int nth, int T);
 cudaError_t launchMppiPrologue(const LaunchArgs& a, int nInst, size_t smem);
 cudaError_t launchMppiRollout(const LaunchArgs& a, int nopp, int nth, bool spl, size_t smem);

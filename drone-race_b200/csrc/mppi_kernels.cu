@@ -6,8 +6,9 @@
 //                   verification histograms.
 //   mppi_rollout    fused perturbation draw + rollout + running/terminal cost + branch
 //                   bookkeeping (fullRolloutKernel, kernels.cu:34-171) + per-branch cost
-//                   aggregation (aggregateBranchCostsKernel, kernels.cu:175-217). One
-//                   thread per (sample, hypothesis); the state stays in registers; the
+//                   aggregation (aggregateBranchCostsKernel, kernels.cu:175-217). Two
+//                   lanes (one opponent) or one thread (two) per (sample, hypothesis); the
+//                   state stays in registers; the
 //                   track, the control sequence and the spline basis are staged in shared
 //                   memory by bulk copies; the perturbation is drawn from Philox instead of
 //                   being read from a stored noise tensor.
@@ -25,21 +26,27 @@
 #include "common.cuh"
 #include "instance.cuh"
 #include "launch.h"
+#include "pair_model.cuh"
 
 namespace dr
 {
 
-// Rollout block size: RB / n_theta samples a CTA, one thread per (sample, hypothesis), up
-// to 128 registers a thread. 256: a rollout CTA takes the registers of one verification
-// CTA, so in the overlapped step the SMs that hold one run one verification CTA beside it
-// (128 CTAs for 4 x 4096 x 2 threads; 1.53 against 1.55 ms per step with 128-thread CTAs,
-// which spread over every SM; 512-thread CTAs: 1.55 ms, the rollout alone 0.39 against
-// 0.32 ms).
+// Rollout block size. With one opponent a CTA is RB / 2 pairs of lanes, one per (sample,
+// hypothesis) (rolloutTilePair); with two it is one thread per (sample, hypothesis).
 #ifndef DR_ROLLOUT_BLOCK
 #define DR_ROLLOUT_BLOCK 256
 #endif
 constexpr int RB = DR_ROLLOUT_BLOCK;
-constexpr int RB_MIN_BLOCKS = RB <= 128 ? 4 : 512 / RB; // register budget of 128 a thread
+// CTAs per SM that the register allocation is sized for. A lane of a pair holds one
+// agent's state: 64 registers a thread (4 CTAs) up to two hypotheses, 80 (3 CTAs) for four
+// and eight, whose actions and beliefs spill 150 to 280 bytes at 64; 128 for two opponents.
+// Measured (B200, 1965 MHz; the rollouts of the engine's front-end settings, K 65536 x 2 x T
+// 80 spline controls / of two agents of K 3001 x 8 x T 61): 2 CTAs 1.48 / 0.94 ms, 3 CTAs
+// 1.34 / 0.86, 4 CTAs 1.26 / 1.04.
+template <int NOPP, int NTH> constexpr int rolloutMinBlocks()
+{
+    return NOPP == 1 ? (NTH <= 2 ? 4 : 3) : 512 / RB;
+}
 // Verification CTAs per SM that the register allocation is sized for (VERIFY_TILE = 512
 // threads a CTA: 2 -> 64 registers a thread). Measured on the 4 x 2^17 x 40 verification
 // of both plans (B200, 1965 MHz), exact arithmetic and a CTA barrier every step:
@@ -148,7 +155,8 @@ struct RolloutSmem
     size_t env, grids, knots, B, vbuf, red, total;
 };
 
-__host__ __device__ inline RolloutSmem rolloutLayout(int nbp, int T, int M, bool spl)
+// cols: columns of the spline buffer (a thread's, or a lane pair's, perturbed knots)
+__host__ __device__ inline RolloutSmem rolloutLayout(int nbp, int T, int M, bool spl, int cols)
 {
     auto a16 = [](size_t x) { return (x + 15) & ~(size_t)15; };
     RolloutSmem L;
@@ -164,7 +172,7 @@ __host__ __device__ inline RolloutSmem rolloutLayout(int nbp, int T, int M, bool
         off = a16(off + (size_t)T * M * 4);
     L.vbuf = off;
     if (spl)
-        off = a16(off + (size_t)M * 2 * RB * 4);
+        off = a16(off + (size_t)M * 2 * cols * 4);
     L.red = off;
     off = a16(off + RB * 4);
     L.total = off;
@@ -335,8 +343,184 @@ __device__ __forceinline__ void rolloutTile(const MppiDev& D, const MppiIn& I, c
     }
 }
 
+// One rollout tile with one opponent: a pair of lanes per (sample, hypothesis), the ego's
+// lane and the opponent's (pair_model.cuh); RB / 2 pairs a CTA. The rollout is bound by the
+// latency of its T dependent steps until the batch fills the device, and by instruction
+// issue and divergence (samples that end early leave their lanes idle) from there. Against a
+// thread per (sample, hypothesis), which moved both agents one after the other (B200, 1965
+// MHz): one agent of K 1024 x 2 x T 50 0.23 -> 0.15 ms, four agents of K 4096 x 2 x T 64
+// 0.32 -> 0.21 alone, one of K 65536 x 2 x T 80 with spline controls 1.45 -> 1.26.
+template <int NTH, bool SPL, bool LOCK>
+__device__ __forceinline__ void rolloutTilePair(const MppiDev& D, const MppiIn& I, const Tile& tile, int K, int T, int M, const EnvParams& E,
+                                                const float* sGrid, const float* sKn, const float* sB, float* vbuf, float* red)
+{
+    constexpr int PAIRS = RB / 2;
+    const Track tr = trackIn(sGrid);
+    const int role = threadIdx.x & 1, pair = threadIdx.x >> 1;
+    const int th = pair % NTH;
+    const int sl = pair / NTH;
+    const int s = tile.s0 + sl;
+    const bool valid = sl < tile.count;
+    const float minConf = D.cfg.minConf;
+    const uint32_t k0 = D.cfg.k0, k1 = D.cfg.k1, step = I.step;
+    const float sig0 = D.cfg.sigma0, sig1 = D.cfg.sigma1;
+
+    BState<NTH> bs;
+#pragma unroll
+    for (int i = 0; i < NTH; i++)
+        bs.belief[i] = I.belief[i];
+    // initBranchState (state.h:154-163)
+    const int pt0 = findConfident<NTH>(bs.belief, minConf);
+    bs.predTheta = pt0;
+    bs.branchingTime = pt0 == 0 ? -1 : 0;
+    const bool compatible = (pt0 == 0 || pt0 == th + 1);
+    bool active = valid && compatible;
+    float cost = active ? 0.0f : INFINITY;
+    DState<1> st;
+    st.pos[0] = I.state.pos[2 * role];
+    st.pos[1] = I.state.pos[2 * role + 1];
+    st.vel[0] = I.state.vel[2 * role];
+    st.vel[1] = I.state.vel[2 * role + 1];
+    st.S[0] = I.state.S[role];
+    st.lat[0] = I.state.lat_dist[role];
+    st.laps[0] = I.state.laps[role];
+    st.locate(E.trackLength);
+    float decay = 1.0f;
+    int tOrigin = 0, curB = -1;
+    for (int t = 0; t < T; t++)
+    {
+        if constexpr (LOCK)
+        {
+            // every thread of the CTA takes this barrier once per step (T is uniform),
+            // keeping the warps on the same step
+            if (!__syncthreads_or(active))
+                break;
+        }
+        // the lanes still rolling out: whole pairs, since both lanes of one decide alike
+        const unsigned mask = __ballot_sync(0xffffffffu, active);
+        if (mask == 0u)
+        {
+            if constexpr (LOCK)
+                continue;
+            else
+                break;
+        }
+        if (!active)
+            continue;
+        const int local = t - tOrigin;
+        const int b = bs.predTheta;
+        const bool oppNoise = E.actionNoise[th][0] != 0.0f;
+        PairNoise noise{k0, k1, (uint32_t)s, ((uint32_t)th << 16) | (uint32_t)t, step, S_MPPI_ROLL_ENV};
+        float ctl0, ctl1, opp0 = 0.0f, opp1 = 0.0f;
+        if constexpr (SPL)
+        {
+            if (oppNoise)
+            {
+                const U4 r = draw(k0, k1, (uint32_t)s, noise.c1, step, S_MPPI_ROLL_ENV, 0);
+                const float2 n = normal_pair_ool(r.x, r.y);
+                opp0 = n.x;
+                opp1 = n.y;
+            }
+            if (b != curB)
+            {
+                // nominal + perturbation of this sample's knots for branch b, the lanes
+                // taking every other knot
+                for (int m = role; m < M; m += 2)
+                {
+                    U4 r = draw(k0, k1, (uint32_t)s, (uint32_t)(b * M + m), step, S_MPPI_EPS, 0);
+                    float e0 = scaled_normal(sig0, r.x);
+                    float e1 = scaled_normal(sig1, r.y);
+                    vbuf[(m * PAIRS + pair) * 2 + 0] = sKn[(b * M + m) * 2 + 0] + e0;
+                    vbuf[(m * PAIRS + pair) * 2 + 1] = sKn[(b * M + m) * 2 + 1] + e1;
+                }
+                curB = b;
+            }
+            __syncwarp(mask);
+            // a lane evaluates one axis of the control
+            const float* Brow = sB + local * M;
+            float sum = 0.0f;
+            for (int m = 0; m < M; m++)
+                sum += Brow[m] * vbuf[m * 2 * PAIRS + threadIdx.x];
+            pairBoth(mask, role, sum, ctl0, ctl1);
+        }
+        else
+        {
+            // the ego's lane draws its perturbation, the opponent's lane its action noise
+            const U4 r = draw(k0, k1, (uint32_t)s, role ? noise.c1 : (uint32_t)(b * T + local), step, role ? S_MPPI_ROLL_ENV : S_MPPI_EPS, 0);
+            opp0 = normal_from_word(r.x);
+            opp1 = normal_from_word(r.y);
+            ctl0 = sKn[(b * T + local) * 2] + __fmul_rn(sig0, opp0);
+            ctl1 = sKn[(b * T + local) * 2 + 1] + __fmul_rn(sig1, opp1);
+        }
+        bool branched = false;
+        const StepOut o = pairStep<NTH>(mask, role, t, th, tr, E, ctl0, ctl1, opp0, opp1, st, bs, branched, minConf, noise);
+        if (branched)
+            tOrigin = t + 1;
+        if (o.term != TERM_NONE)
+            active = false;
+        cost += stateCost(o, E, D.cfg.w) * decay;
+        decay *= DECAY;
+    }
+    {
+        DState<2> both; // the final cost reads both agents' arc lengths and laps
+        pairBoth(0xffffffffu, role, st.S[0], both.S[0], both.S[1]);
+        pairBoth(0xffffffffu, role, st.laps[0], both.laps[0], both.laps[1]);
+        if (valid && compatible)
+            cost += finalCost<1>(both, E, D.cfg.w.finalAdvWeight, D.cfg.w.finalOppAdvWeight);
+    }
+    if (valid && role == 0)
+    {
+        D.costsTrue[th * K + s] = cost;
+        D.binfo[th * K + s] = packInfo(bs.predTheta, bs.branchingTime);
+        if (compatible && !isfinite(cost))
+            atomicAdd(&D.stats[0], 1);
+    }
+    if (role == 0)
+        red[pair] = cost;
+    __syncthreads();
+    // aggregateBranchCostsKernel (kernels.cu:175-217): costs[b][s] = E_belief[cost | b]
+    if (valid)
+    {
+        const float* c = red + sl * NTH;
+        if (role == 0)
+        {
+            float num = 0.0f, den = 0.0f;
+            float cv = c[th];
+            if (isfinite(cv))
+            {
+                float w = I.belief[th];
+                num += w * cv;
+                den += w;
+            }
+            D.costs[(size_t)(th + 1) * K + s] = (den > 1e-30f) ? (num / den) : INFINITY;
+        }
+        else if (th == 0)
+        {
+            float num = 0.0f, den = 0.0f;
+#pragma unroll
+            for (int m = 0; m < NTH; m++)
+            {
+                float cv = c[m];
+                if (!isfinite(cv))
+                    continue;
+                float w = I.belief[m];
+                num += w * cv;
+                den += w;
+            }
+            D.costs[s] = (den > 1e-30f) ? (num / den) : INFINITY;
+        }
+    }
+}
+
+// CTAs that share a tile of the table (rolloutSamplesPerBlock samples): a CTA of lane pairs
+// takes half the samples that one of single threads does.
+template <int NOPP> constexpr int rolloutParts()
+{
+    return NOPP == 1 ? 2 : 1;
+}
+
 template <int NOPP, int NTH, bool SPL, bool PQ, bool LOCK>
-__global__ void __launch_bounds__(RB, RB_MIN_BLOCKS) mppi_rollout(const MppiDev* __restrict__ insts, const MppiIn* __restrict__ in,
+__global__ void __launch_bounds__(RB, (rolloutMinBlocks<NOPP, NTH>())) mppi_rollout(const MppiDev* __restrict__ insts, const MppiIn* __restrict__ in,
                                                                        const Tile* __restrict__ tiles, int nTiles, unsigned* __restrict__ queue)
 {
     constexpr int NBP = NTH + 1;
@@ -351,13 +535,21 @@ __global__ void __launch_bounds__(RB, RB_MIN_BLOCKS) mppi_rollout(const MppiDev*
     for (int iter = 0;; iter++)
     {
         const int ti = nextTile(PQ ? queue : nullptr, iter, &sTicket);
-        if (ti >= nTiles)
+        constexpr int PARTS = rolloutParts<NOPP>();
+        if (ti >= nTiles * PARTS)
             break;
-        const Tile tile = tiles[ti];
+        Tile tile = tiles[ti / PARTS];
+        if constexpr (PARTS > 1)
+        {
+            constexpr int PER = RB / NTH / PARTS;
+            const int part = ti % PARTS;
+            tile.s0 += part * PER;
+            tile.count = min(max(tile.count - part * PER, 0), PER);
+        }
         const MppiDev& D = insts[tile.inst];
         const MppiIn& I = in[tile.inst];
         const int K = D.cfg.K, T = D.cfg.T, M = D.cfg.M;
-        const RolloutSmem L = rolloutLayout(NBP, T, M, SPL);
+        const RolloutSmem L = rolloutLayout(NBP, T, M, SPL, RB / PARTS);
         EnvParams* sE = (EnvParams*)(smraw + L.env);
         float* sGrid = (float*)(smraw + L.grids);
         float* sKn = (float*)(smraw + L.knots);
@@ -393,7 +585,10 @@ __global__ void __launch_bounds__(RB, RB_MIN_BLOCKS) mppi_rollout(const MppiDev*
             phase ^= 1u;
             staged = tile.inst;
         }
-        rolloutTile<NOPP, NTH, SPL, LOCK>(D, I, tile, K, T, M, *sE, sGrid, sKn, sB, vbuf, red);
+        if constexpr (NOPP == 1)
+            rolloutTilePair<NTH, SPL, LOCK>(D, I, tile, K, T, M, *sE, sGrid, sKn, sB, vbuf, red);
+        else
+            rolloutTile<NOPP, NTH, SPL, LOCK>(D, I, tile, K, T, M, *sE, sGrid, sKn, sB, vbuf, red);
         __syncthreads(); // the next tile's staging and reduction buffer reuse shared memory
     }
 }
@@ -1086,9 +1281,9 @@ __global__ void mppi_noise(const MppiDev* __restrict__ insts, const MppiIn* __re
 // ---------------------------------------------------------------------------------------
 // dispatch
 // ---------------------------------------------------------------------------------------
-size_t mppiRolloutSmem(int nth, int T, int M, bool spl)
+size_t mppiRolloutSmem(int nopp, int nth, int T, int M, bool spl)
 {
-    return rolloutLayout(nth + 1, T, M, spl).total;
+    return rolloutLayout(nth + 1, T, M, spl, nopp == 1 ? RB / rolloutParts<1>() : RB).total;
 }
 
 size_t mppiVerifySmem(int nth, int T)
@@ -1101,7 +1296,8 @@ template <int NOPP, int NTH, bool SPL> static cudaError_t launchRolloutS(const L
     auto k = a.queue ? (a.lockstep ? mppi_rollout<NOPP, NTH, SPL, true, true> : mppi_rollout<NOPP, NTH, SPL, true, false>)
                      : (a.lockstep ? mppi_rollout<NOPP, NTH, SPL, false, true> : mppi_rollout<NOPP, NTH, SPL, false, false>);
     ensureSmem(k, smem);
-    k<<<launchGrid(a), RB, smem, a.stream>>>(a.mppi, a.mppiIn, a.tiles, a.nTiles, a.queue);
+    const int work = a.nTiles * rolloutParts<NOPP>();
+    k<<<a.queue && a.grid < work ? a.grid : work, RB, smem, a.stream>>>(a.mppi, a.mppiIn, a.tiles, a.nTiles, a.queue);
     return cudaGetLastError();
 }
 

@@ -195,7 +195,7 @@ extern "C" int dr_mppi_rollout_costs_noalloc(const dr_env_config* env, const dr_
     a.mppiIn = (const MppiIn*)(base + oIn);
     a.tiles = (const Tile*)(base + oTiles);
     a.nTiles = nTiles;
-    CK(launchMppiRollout(a, env->n_opp, nth, spl, mppiRolloutSmem(nth, T, M, spl)));
+    CK(launchMppiRollout(a, env->n_opp, nth, spl, mppiRolloutSmem(env->n_opp, nth, T, M, spl)));
     // copies from pageable host memory have taken their data when they return, so the
     // host records may go out of scope; wait for the kernel so that the caller may read
     // costs_dev on any stream afterwards
