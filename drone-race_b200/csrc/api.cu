@@ -1077,9 +1077,13 @@ static int createMppi(const dr_env_config* env, const dr_gate_env_config* genv, 
     A.add(cpTab, sizeof(double) * 3 * CP_TAB);
     // the ego tables of the fast verification (strategic race), when they stay small
     EgoRow* egoTab = nullptr;
+    float* clear = nullptr;
     const size_t egoBytes = (size_t)2 * egoRows(nth, h->H) * h->H * sizeof(EgoRow);
     if (env && cfg->verify && egoBytes <= EGO_TABLE_MAX_BYTES)
+    {
         A.add(egoTab, egoBytes);
+        A.add(clear, (size_t)2 * clearWords(h->H) * 4);
+    }
 
     // result block, one contiguous range
     size_t oFail = 0, oDense = a16(oFail + (size_t)2 * T * 4), oPrev = oDense + a16((size_t)nbp * T * 2 * 4), oNu = oPrev + a16((size_t)nbp * T * 2 * 4),
@@ -1120,6 +1124,7 @@ static int createMppi(const dr_env_config* env, const dr_gate_env_config* genv, 
     D.minCosts = minCosts;
     D.stats = stats;
     D.egoTab = egoTab;
+    D.clear = clear;
     D.resBytes = resBytes;
     if (env)
     {
@@ -1787,6 +1792,8 @@ static int debugVerify(dr_mppi* h, const St* state, const float* belief, const f
         a.nTiles = (int)tiles.size();
         a.exactVerify = h->exactVerify ? 1 : 0;
         a.egoTable = h->envKind == 0 && h->egoTableUsable() ? 1 : 0;
+        if (a.egoTable) // the prologue zeroes the clearance blocks in a step
+            cudaMemsetAsync(D.clear, 0, (size_t)2 * clearWords(h->H) * 4, h->stream);
         if (a.egoTable)
             e = launchEgoTable(h->stream, h->nopp, h->nth, dD, dIn, 1, plan, h->H);
         if (e == cudaSuccess)

@@ -83,6 +83,7 @@ struct MppiDev
     // samples (EgoRow): [plan][row][H], row 0 = no branch (or the branch of a confident
     // initial belief), row 1 + (b - 1) H + tb = branch b taken at step tb; or null
     EgoRow* egoTab;
+    float* clear; // [plan][clearWords(H)]: the ego's whereabouts under each plan (ClearBlock), with egoTab
     size_t resBytes;
 };
 
@@ -93,6 +94,38 @@ __host__ __device__ __forceinline__ int egoRows(int nth, int H)
 {
     return 1 + nth * H;
 }
+
+// Where the ego can be under a plan, from its ego table: for the verification's proof that
+// no remaining step of a sample can collide (clearOfEgo). Floats, zeroed by the prologue and
+// filled by mppi_ego_table, in order:
+//   xy [H][2]    the ego's position after each step on the trajectory with no branch
+//   all [H]      the largest distance from there, after each step, over the trajectories that
+//                branch; infinite where one of them is off the track
+//   out          nonzero when the trajectory with no branch leaves the track
+//   rho [G][H]   as `all`, over those that branch within group g's steps (clearPer(H) a group)
+constexpr int CLEAR_GROUPS = 40; // most groups; longer horizons put several steps in one
+
+__host__ __device__ __forceinline__ int clearPer(int H)
+{
+    return (H + CLEAR_GROUPS - 1) / CLEAR_GROUPS;
+}
+
+__host__ __device__ __forceinline__ int clearGroups(int H)
+{
+    return (H + clearPer(H) - 1) / clearPer(H);
+}
+
+// floats of one plan's block, a multiple of 4 (16-byte bulk copies)
+__host__ __device__ __forceinline__ int clearWords(int H)
+{
+    return (3 * H + 1 + clearGroups(H) * H + 3) & ~3;
+}
+
+template <class F> struct ClearBlock
+{
+    F *xy, *all, *out, *rho;
+    __device__ __forceinline__ ClearBlock(F* p, int H) : xy(p), all(p + 2 * H), out(p + 3 * H), rho(p + 3 * H + 1) {}
+};
 
 struct PrCfgDev
 {

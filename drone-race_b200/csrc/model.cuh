@@ -506,29 +506,6 @@ __device__ __forceinline__ float projectOnTrack(const Track& tr, float L, float 
     return projectSegments<F>(tr, L, invL, px, py, bestJ, latDist, tpS);
 }
 
-// projectOnTrack<true> with the window scan spread over the 32 lanes of a warp, all of
-// which hold the same position and take part: lane j < 21 evaluates window sample j and one
-// warp-wide unsigned minimum of the packed (squared distance, place) keys finds the nearest;
-// every lane returns projectOnTrack<true>'s result.
-__device__ __forceinline__ float projectOnTrackWarp(const Track& tr, float L, float invL, float px, float py, float prevS, float& latDist, TrackPos& tpS)
-{
-    prevS *= invL;
-    prevS = prevS - floorf(prevS);
-    const int idxPrev = (int)(prevS * NTS);
-    const int j0 = idxPrev - WIN;
-    const uint32_t lane = threadIdx.x & 31u;
-    uint32_t key = 0xffffffffu;
-    if (lane <= 2 * WIN)
-    {
-        const int j = j0 + (int)lane;
-        const float d0 = __fsub_rn(tr.px[j], px), d1 = __fsub_rn(tr.py[j], py);
-        const float sq = __fmaf_rn(d1, d1, __fmul_rn(d0, d0));
-        key = (__float_as_uint(sq) & ~31u) | lane;
-    }
-    key = __reduce_min_sync(0xffffffffu, key);
-    return projectSegments<true>(tr, L, invL, px, py, j0 + (int)(key & 31u), latDist, tpS);
-}
-
 // ---- per-step agent quantities -------------------------------------------------------
 
 template <int NA> struct AgentGeo
@@ -785,9 +762,9 @@ struct __align__(16) EgoRow
 };
 
 // The ego's part of envStep (geometry, clamp, position, arc length, velocity, speed cap,
-// projection, laps; the same expressions), for an ego that draws no noise. WARP (fast
-// flavour only): all 32 lanes of the warp hold the same ego and share the projection's scan.
-template <bool F, bool WARP = false>
+// projection, laps; the same expressions), for an ego that draws no noise. CLAMPED: the
+// action is within the acceleration limit already.
+template <bool F, bool CLAMPED = false>
 __device__ __forceinline__ void egoStep(const Track& tr, const EnvParams& E, float ego0, float ego1, DState<1>& s, EgoRow& row)
 {
     AgentGeo<1> g;
@@ -796,15 +773,18 @@ __device__ __forceinline__ void egoStep(const Track& tr, const EnvParams& E, flo
     row.tn1 = g.tn1[0];
     row.sdot = g.sdot[0];
     const float prevS = s.S[0];
-    float sq = 0.0f;
-    sq += ego0 * ego0;
-    sq += ego1 * ego1;
-    float factor = 1.0f;
-    float maxSq = E.maxAccel[0] * E.maxAccel[0];
-    if (sq > maxSq)
-        factor = mdivsqrt<F>(E.maxAccel[0], sq);
-    ego0 *= factor;
-    ego1 *= factor;
+    if constexpr (!CLAMPED)
+    {
+        float sq = 0.0f;
+        sq += ego0 * ego0;
+        sq += ego1 * ego1;
+        float factor = 1.0f;
+        float maxSq = E.maxAccel[0] * E.maxAccel[0];
+        if (sq > maxSq)
+            factor = mdivsqrt<F>(E.maxAccel[0], sq);
+        ego0 *= factor;
+        ego1 *= factor;
+    }
     s.pos[0] += E.dt * s.vel[0];
     s.pos[1] += E.dt * s.vel[1];
     s.S[0] += E.dt * g.sdot[0];
@@ -817,10 +797,7 @@ __device__ __forceinline__ void egoStep(const Track& tr, const EnvParams& E, flo
         s.vel[0] *= sc;
         s.vel[1] *= sc;
     }
-    if constexpr (WARP)
-        s.S[0] = projectOnTrackWarp(tr, E.trackLength, E.invTrackLength, s.pos[0], s.pos[1], s.S[0], s.lat[0], s.tp[0]);
-    else
-        s.S[0] = projectOnTrack<F>(tr, E.trackLength, E.invTrackLength, s.pos[0], s.pos[1], s.S[0], s.lat[0], s.tp[0]);
+    s.S[0] = projectOnTrack<F>(tr, E.trackLength, E.invTrackLength, s.pos[0], s.pos[1], s.S[0], s.lat[0], s.tp[0]);
     if (s.S[0] < prevS - E.trackLength * 0.5f)
         s.laps[0]++;
     if (s.S[0] > prevS + E.trackLength * 0.5f)

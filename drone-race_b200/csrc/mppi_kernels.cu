@@ -20,6 +20,7 @@
 //                   the spline interpolation and the clamp (kernels.cu:411-456).
 //   mppi_verify     Monte-Carlo failure counts of the new and the previous plan
 //                   (verifyNominalFailureKernel, kernels.cu:488-551), both plans in one grid.
+#include <cfloat>
 #include <cstdio>
 #include <type_traits>
 
@@ -77,12 +78,15 @@ __device__ __forceinline__ int infoTime(int v)
 }
 
 // Copies the host-filled part of EnvParams to shared memory and computes the
-// device-filled part; the caller's next __syncthreads publishes both.
+// device-filled part from there (from global memory its dependent reads were a chain of L2
+// latencies at the start of every kernel); all threads of the CTA, and the caller's next
+// __syncthreads publishes the terms.
 __device__ __forceinline__ void copyEnv(EnvParams* dst, const EnvParams* src)
 {
     for (int i = threadIdx.x; i < ENV_HOST_WORDS; i += blockDim.x)
         ((float*)dst)[i] = ((const float*)src)[i];
-    envDeviceTerms(*dst, *src, threadIdx.x, blockDim.x);
+    __syncthreads();
+    envDeviceTerms(*dst, *dst, threadIdx.x, blockDim.x);
 }
 
 __host__ __device__ __forceinline__ size_t align16(size_t x)
@@ -106,6 +110,9 @@ __global__ void __launch_bounds__(256) mppi_prologue(const MppiDev* __restrict__
         D.fail[i] = 0u;
     if (threadIdx.x < 4)
         D.stats[threadIdx.x] = 0;
+    if (D.clear)
+        for (int i = threadIdx.x; i < 2 * clearWords(D.cfg.H) / 4; i += blockDim.x)
+            reinterpret_cast<float4*>(D.clear)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     const int b = I.pendBranch;
     if (b < 0 || b >= nbp)
         return;
@@ -1025,20 +1032,119 @@ __global__ void __launch_bounds__(UB) mppi_shard_apply(const MppiDev* __restrict
 // ---------------------------------------------------------------------------------------
 // verification
 // ---------------------------------------------------------------------------------------
-// The ego tables of a plan (EgoRow; plan 0 the new one, 1 the previous one, 2 both): one
-// warp per row (the trajectory with no branch, and one per branch and branching step)
-// moves the ego alone through the verification horizon with the fast arithmetic of the
-// verification, its lanes sharing the projection's window scan; each CTA of
+// The ego tables of a plan (EgoRow; plan 0 the new one, 1 the previous one, 2 both): a row
+// is the trajectory with no branch, or the one of a branch and a branching step, moved alone
+// through the verification horizon with the fast arithmetic of the verification; each CTA of
 // EGO_WARPS warps stages the track, the environment and the plan in shared memory. The
-// rows are independent, so the kernel's time is one trajectory's: H steps of one warp.
+// kernel's time is one row's chain of H steps. Only position and velocity need that chain,
+// and they do not need the track: so EGO_STEPS lanes take as many steps of a row, each lane
+// runs the short chain up to its own step and then projects that position by itself, from the
+// sample that the steps before ended at. The sample found is the one that the window scan of
+// the step-by-step projection finds wherever the certificate holds there and the sample lies
+// in that step's window, which the lane checks once its neighbour's arc length is known; where
+// it does not, the steps are taken one by one (egoStep). The lane also runs the trajectory
+// with no branch beside its own and puts its distance from it into the clearance block.
 constexpr int EGO_WARPS = 4;
+// Steps between two clearance tests of a verification warp: a test costs about 60
+// instructions, a step about 700. Four agents of 2 x 2^17 x 40, three drawn mid-race states
+// (B200, 1965 MHz; the verification of the new plan): without the test 0.52 / 0.45 / 0.55 ms,
+// every step 0.36 / 0.27 / 0.08, every second 0.35 / 0.26 / 0.08, every fourth 0.35 / 0.25 /
+// 0.10.
+#ifndef DR_CLEAR_EVERY
+#define DR_CLEAR_EVERY 2
+#endif
+constexpr int CLEAR_EVERY = DR_CLEAR_EVERY;
+
+// Whether no remaining step (t .. H - 1) of the warp's active samples can bring an opponent
+// within two drone radii of the ego, or the ego off the track: then none of them can fail any
+// more (a sample fails at the first step with boundary distance below the drone radius) and
+// their remaining steps decide nothing. px .. vy: this lane's opponent before step t; xy: the
+// ego's trajectory with no branch (which stays on the track), rho: how far the samples' own may
+// be from it, after each step.
+//
+// An opponent whose speed is within its limit vmax moves k dt v in k steps plus at most
+// amax dt^2 k (k - 1) / 2: the step moves it by its velocity before the step and then adds an
+// acceleration clamped to amax, and the cap to vmax, a projection onto a ball that holds the
+// old velocity, never moves the new one farther from it. The warp's opponents lie within
+// (dp, dv) of the first active lane's in position and velocity (1-norms, which bound the
+// Euclidean ones). The ego is on a row of its table: within rho of the trajectory with no
+// branch. So after step j the two are at least |ego_j - (p + k dt v)| - rho - dp - k dt dv -
+// amax dt^2 k (k - 1) / 2 apart, k = j - t + 1. Slack for the arithmetic (the verification's
+// approximate factors are within 1e-5, positions round to 2^-24 a step): a millimetre, 1e-4 of
+// the reach and of the speed limit's way, and H roundings of the coordinates.
+__device__ __forceinline__ bool clearOfEgo(const EnvParams& E, const float* xy, const float* rho, int H, int t, bool active, float px, float py, float vx,
+                                           float vy, float vmax, float amax)
+{
+    vmax = fabsf(vmax);
+    amax = fabsf(amax);
+    constexpr unsigned ALL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int src = __ffs(__ballot_sync(ALL, active)) - 1;
+    const float cx = __shfl_sync(ALL, px, src), cy = __shfl_sync(ALL, py, src), wx = __shfl_sync(ALL, vx, src), wy = __shfl_sync(ALL, vy, src);
+    float dp = 0.0f, dv = 0.0f;
+    bool ok = true;
+    if (active)
+    {
+        dp = fabsf(px - cx) + fabsf(py - cy);
+        dv = fabsf(vx - wx) + fabsf(vy - wy);
+        ok = vx * vx + vy * vy <= vmax * vmax * 1.0001f;
+    }
+    // non-negative floats (and NaN, above them all) order as their words
+    dp = __uint_as_float(__reduce_max_sync(ALL, __float_as_uint(dp)));
+    dv = __uint_as_float(__reduce_max_sync(ALL, __float_as_uint(dv)));
+    for (int j = t + lane; j < H; j += 32)
+    {
+        const float k = (float)(j - t + 1), kd = k * E.dt;
+        const float ex = xy[2 * j] - (cx + kd * wx), ey = xy[2 * j + 1] - (cy + kd * wy);
+        const float way = kd * vmax;
+        const float reach = 2.0f * E.droneRadius + rho[j] + dp + kd * dv + 0.5f * amax * E.dt * E.dt * (k * (k - 1.0f));
+        const float slack = 1e-3f + 1e-4f * (reach + way) + 2.4e-7f * (float)H * (fabsf(cx) + fabsf(cy) + way);
+        const float need = reach + slack;
+        ok = ok && ex * ex + ey * ey > need * need;
+    }
+    return __all_sync(ALL, ok);
+}
+
+// 8 / 16 / 32 steps at a time: 18.5 / 17.0 / 16.6 us for a plan of four agents, H 40, two
+// hypotheses (B200, 1965 MHz); more steps repeat more of the short chain, which large batches
+// pay for. A warp per row, step by step, its lanes sharing the window scan: 31 us, without
+// the clearance block.
+#ifndef DR_EGO_STEPS
+#define DR_EGO_STEPS 16
+#endif
+constexpr int EGO_STEPS = DR_EGO_STEPS;                  // steps of a row taken at a time, a lane each
+constexpr int EGO_CTA_ROWS = EGO_WARPS * 32 / EGO_STEPS; // rows a CTA takes at a time
+
+// The squared distance from (px, py) to track sample i (0 .. 511).
+__device__ __forceinline__ float sampleSqDist(const Track& tr, int i, float px, float py)
+{
+    const float dx = tr.px[i] - px, dy = tr.py[i] - py;
+    return dx * dx + dy * dy;
+}
+
+// egoStep's position, velocity and speed cap under a control already clamped
+__device__ __forceinline__ void egoAdvance(const EnvParams& E, const float* ctl, float (&p)[2], float (&v)[2])
+{
+    p[0] += E.dt * v[0];
+    p[1] += E.dt * v[1];
+    v[0] += E.dt * ctl[0];
+    v[1] += E.dt * ctl[1];
+    float sqSpd = sqNorm(v[0], v[1]);
+    if (sqSpd > E.maxSpeed[0] * E.maxSpeed[0])
+    {
+        float sc = mdivsqrt<true>(E.maxSpeed[0], sqSpd);
+        v[0] *= sc;
+        v[1] *= sc;
+    }
+}
 
 template <int NTH>
 __global__ void __launch_bounds__(EGO_WARPS * 32) mppi_ego_table(const MppiDev* __restrict__ insts, const MppiIn* __restrict__ in, int nInst, int plans)
 {
-    __shared__ float sg[GRID_FLOATS];
-    __shared__ __align__(16) float sPlan[(DR_MAX_THETA + 1) * DR_MAX_T * 2];
+    __shared__ __align__(16) float sg[GRID_FLOATS];
+    __shared__ __align__(16) float sPlan[(NTH + 1) * DR_MAX_T * 2];
     __shared__ EnvParams sE;
+    __shared__ __align__(8) uint64_t bar;
     const int inst = blockIdx.x;
     if (inst >= nInst)
         return;
@@ -1047,9 +1153,15 @@ __global__ void __launch_bounds__(EGO_WARPS * 32) mppi_ego_table(const MppiDev* 
     if (!D.egoTab)
         return;
     const int H = D.cfg.H, T = D.cfg.T, rows = egoRows(NTH, H), nbp = NTH + 1;
-    const int warp = threadIdx.x >> 5;
-    for (int i = threadIdx.x; i < GRID_FLOATS; i += blockDim.x)
-        sg[i] = D.grids[i];
+    const int p0 = plans == 1 ? 1 : 0, p1 = plans == 0 ? 0 : 1;
+    const uint32_t planBytes = (uint32_t)align16((size_t)nbp * T * 2 * 4);
+    if (threadIdx.x == 0)
+    {
+        mbar_init(&bar, 1);
+        mbar_expect_tx(&bar, GRID_FLOATS * 4 + planBytes);
+        bulk_g2s(sg, D.grids, GRID_FLOATS * 4, &bar);
+        bulk_g2s(sPlan, p0 == 0 ? D.dense : D.prevDense, planBytes, &bar);
+    }
     copyEnv(&sE, &D.env);
     const EnvParams& E = sE;
     const Track tr = trackIn(sg);
@@ -1058,23 +1170,55 @@ __global__ void __launch_bounds__(EGO_WARPS * 32) mppi_ego_table(const MppiDev* 
     for (int i = 0; i < NTH; i++)
         belief[i] = I.belief[i];
     const int pt0 = findConfident<NTH>(belief, D.cfg.minConf);
-    const int p0 = plans == 1 ? 1 : 0, p1 = plans == 0 ? 0 : 1;
+    const int sub = threadIdx.x % EGO_STEPS; // this lane's step
+    constexpr unsigned ALL = 0xffffffffu;
     for (int plan = p0; plan <= p1; plan++)
     {
-        const float* P = plan == 0 ? D.dense : D.prevDense;
-        __syncthreads(); // the previous plan's rows are done with sPlan
-        for (int i = threadIdx.x; i < nbp * T * 2; i += blockDim.x)
-            sPlan[i] = P[i];
-        __syncthreads();
+        __syncthreads(); // the environment's terms, and the previous plan's rows are done with sPlan
+        if (threadIdx.x == 0 && plan != p0)
+        {
+            mbar_expect_tx(&bar, planBytes);
+            bulk_g2s(sPlan, D.prevDense, planBytes, &bar);
+        }
+        if (!__syncthreads_and(mbar_wait(&bar, (uint32_t)(plan - p0))))
+        {
+            // uniform: the step reports the timeout, as for the other kernels' staging
+            if (threadIdx.x == 0)
+                atomicAdd(&D.stats[1], 1);
+            return;
+        }
         if (!egoNoiseFree(E))
             continue; // uniform: the verification moves the ego itself
-        EgoRow* tab = D.egoTab + (size_t)plan * rows * H;
-        for (int r = blockIdx.y * EGO_WARPS + warp; r < rows; r += gridDim.y * EGO_WARPS)
+        // egoStep's clamp of the controls
+        for (int i = threadIdx.x; i < nbp * T; i += blockDim.x)
         {
-            if (r > 0 && pt0 != 0)
-                break; // a confident initial belief never branches
+            float ego0 = sPlan[2 * i], ego1 = sPlan[2 * i + 1];
+            float sq = 0.0f;
+            sq += ego0 * ego0;
+            sq += ego1 * ego1;
+            float factor = 1.0f;
+            float maxSq = E.maxAccel[0] * E.maxAccel[0];
+            if (sq > maxSq)
+                factor = mdivsqrt<true>(E.maxAccel[0], sq);
+            sPlan[2 * i] = ego0 * factor;
+            sPlan[2 * i + 1] = ego1 * factor;
+        }
+        __syncthreads();
+        EgoRow* tab = D.egoTab + (size_t)plan * rows * H;
+        const ClearBlock<float> cb(D.clear + (size_t)plan * clearWords(H), H);
+        const float L = E.trackLength, invL = E.invTrackLength;
+        const int nRows = pt0 != 0 ? 1 : rows; // a confident initial belief never branches
+        // whole warps take part as long as one of their rows exists; the others repeat row 0
+        for (int base = blockIdx.y * EGO_CTA_ROWS; base + (int)(threadIdx.x & ~31u) / EGO_STEPS < nRows; base += gridDim.y * EGO_CTA_ROWS)
+        {
+            const int want = base + (int)threadIdx.x / EGO_STEPS;
+            const bool mine = want < nRows;
+            const int r = mine ? want : 0;
             const int bb = r > 0 ? 1 + (r - 1) / H : 0, tb = r > 0 ? (r - 1) % H : H;
-            DState<1> s;
+            // the verification's plan index: branch pt0 before any branching, then the
+            // branch taken, its clock restarting after the branching step
+            auto control = [&](int t) { return sPlan + ((t <= tb ? pt0 : bb) * T + (t <= tb ? t : t - tb - 1)) * 2; };
+            DState<1> s; // after the steps done, alike on the row's lanes
             s.pos[0] = I.state.pos[0];
             s.pos[1] = I.state.pos[1];
             s.vel[0] = I.state.vel[0];
@@ -1082,21 +1226,146 @@ __global__ void __launch_bounds__(EGO_WARPS * 32) mppi_ego_table(const MppiDev* 
             s.S[0] = I.state.S[0];
             s.lat[0] = I.state.lat_dist[0];
             s.laps[0] = I.state.laps[0];
-            s.locate(E.trackLength);
-            for (int t = 0; t < H; t++)
+            s.locate(L);
+            float bp[2] = {s.pos[0], s.pos[1]}, bv[2] = {s.vel[0], s.vel[1]}; // the trajectory with no branch
+            AgentGeo<1> g; // of s
+            agentGeometry<1, true>(tr, E, s, g);
+            int near = wrapNts(s.tp[0].i0);
+            for (int t0 = 0; t0 < H; t0 += EGO_STEPS)
             {
-                // the verification's plan index: branch pt0 before any branching, then the
-                // branch taken, its clock restarting after the branching step
-                const int b = t <= tb ? pt0 : bb, local = t <= tb ? t : t - tb - 1;
+                const int t = t0 + sub;
+                DState<1> m; // after step t
+                float p[2] = {s.pos[0], s.pos[1]}, v[2] = {s.vel[0], s.vel[1]}, b0 = 0.0f, b1 = 0.0f;
+#pragma unroll 4
+                for (int u = 0; u < EGO_STEPS; u++)
+                {
+                    if (t0 + u < H)
+                    {
+                        egoAdvance(E, control(t0 + u), p, v);
+                        egoAdvance(E, sPlan + (pt0 * T + t0 + u) * 2, bp, bv);
+                    }
+                    if (u <= sub)
+                    {
+                        m.pos[0] = p[0];
+                        m.pos[1] = p[1];
+                        m.vel[0] = v[0];
+                        m.vel[1] = v[1];
+                        b0 = bp[0];
+                        b1 = bp[1];
+                    }
+                }
+                // walk to a local minimum of the distances
+                int c = near;
+                float dc = sampleSqDist(tr, c, m.pos[0], m.pos[1]);
+                const int dir = sampleSqDist(tr, wrapNts(c + 1), m.pos[0], m.pos[1]) < dc ? 1 : NTS - 1;
+                for (int n = 0; n < NTS; n++)
+                {
+                    const int next = wrapNts(c + dir);
+                    const float dn = sampleSqDist(tr, next, m.pos[0], m.pos[1]);
+                    if (!(dn < dc))
+                        break;
+                    c = next;
+                    dc = dn;
+                }
+                m.S[0] = projectSegments<true>(tr, L, invL, m.pos[0], m.pos[1], c, m.lat[0], m.tp[0]);
+                AgentGeo<1> gm;
+                agentGeometry<1, true>(tr, E, m, gm);
+                // the state before step t: the neighbour's, or the one after the steps done
                 EgoRow row;
-                egoStep<true, true>(tr, E, sPlan[(b * T + local) * 2], sPlan[(b * T + local) * 2 + 1], s, row);
-                if ((threadIdx.x & 31) == 0)
+                float pS = __shfl_up_sync(ALL, m.S[0], 1, EGO_STEPS);
+                row.tn0 = __shfl_up_sync(ALL, gm.tn0[0], 1, EGO_STEPS);
+                row.tn1 = __shfl_up_sync(ALL, gm.tn1[0], 1, EGO_STEPS);
+                row.sdot = __shfl_up_sync(ALL, gm.sdot[0], 1, EGO_STEPS);
+                if (sub == 0)
+                {
+                    pS = s.S[0];
+                    row.tn0 = g.tn0[0];
+                    row.tn1 = g.tn1[0];
+                    row.sdot = g.sdot[0];
+                }
+                float q = pS;
+                q += E.dt * row.sdot;
+                q *= invL;
+                q = q - floorf(q);
+                const int j0 = (int)(q * NTS) - WIN;
+                const bool found = dc <= tr.cert[c] && wrapNts(c - j0 + 2 * NTS) <= 2 * WIN;
+                if (__all_sync(ALL, found || t >= H))
+                {
+                    int laps = (m.S[0] < pS - L * 0.5f ? 1 : 0) - (m.S[0] > pS + L * 0.5f ? 1 : 0);
+#pragma unroll
+                    for (int o = 1; o < EGO_STEPS; o *= 2)
+                    {
+                        const int x = __shfl_up_sync(ALL, laps, o, EGO_STEPS);
+                        if (sub >= o)
+                            laps += x;
+                    }
+                    row.pos0 = m.pos[0];
+                    row.pos1 = m.pos[1];
+                    row.vel0 = m.vel[0];
+                    row.vel1 = m.vel[1];
+                    row.S = m.S[0];
+                    row.lat = m.lat[0];
+                    row.w = m.tp[0].w;
+                    row.laps = s.laps[0] + laps;
+                    row.i0 = m.tp[0].i0;
+                    constexpr int LAST = EGO_STEPS - 1;
+                    s.pos[0] = p[0];
+                    s.pos[1] = p[1];
+                    s.vel[0] = v[0];
+                    s.vel[1] = v[1];
+                    s.S[0] = __shfl_sync(ALL, m.S[0], LAST, EGO_STEPS);
+                    s.lat[0] = __shfl_sync(ALL, m.lat[0], LAST, EGO_STEPS);
+                    s.laps[0] = __shfl_sync(ALL, row.laps, LAST, EGO_STEPS);
+                    s.tp[0].i0 = __shfl_sync(ALL, m.tp[0].i0, LAST, EGO_STEPS);
+                    s.tp[0].w = __shfl_sync(ALL, m.tp[0].w, LAST, EGO_STEPS);
+                    g.tn0[0] = __shfl_sync(ALL, gm.tn0[0], LAST, EGO_STEPS);
+                    g.tn1[0] = __shfl_sync(ALL, gm.tn1[0], LAST, EGO_STEPS);
+                    g.sdot[0] = __shfl_sync(ALL, gm.sdot[0], LAST, EGO_STEPS);
+                    near = __shfl_sync(ALL, c, LAST, EGO_STEPS);
+                }
+                else
+                {
+                    for (int u = 0; u < EGO_STEPS && t0 + u < H; u++)
+                    {
+                        const float* ctl = control(t0 + u);
+                        EgoRow step;
+                        egoStep<true, true>(tr, E, ctl[0], ctl[1], s, step);
+                        if (sub == u)
+                            row = step;
+                    }
+                    agentGeometry<1, true>(tr, E, s, g);
+                    near = wrapNts(s.tp[0].i0);
+                }
+                if (mine && t < H)
+                {
                     tab[(size_t)r * H + t] = row;
+                    const bool off = !(E.trackWidth - fabsf(row.lat) >= E.droneRadius);
+                    if (r == 0)
+                    {
+                        cb.xy[2 * t] = row.pos0;
+                        cb.xy[2 * t + 1] = row.pos1;
+                        if (off)
+                            *cb.out = 1.0f;
+                    }
+                    else if (t > tb) // up to its branching step a row is the first one
+                    {
+                        // off the track, or a distance that is no number: infinitely far
+                        const float dx = row.pos0 - b0, dy = row.pos1 - b1;
+                        float d = sqrtf(dx * dx + dy * dy);
+                        if (off || !(d <= FLT_MAX))
+                            d = INFINITY;
+                        // distances are not negative: they order as their words
+                        atomicMax((unsigned*)&cb.all[t], __float_as_uint(d));
+                        atomicMax((unsigned*)&cb.rho[tb / clearPer(H) * H + t], __float_as_uint(d));
+                    }
+                }
             }
         }
     }
 }
 
+// What bounds it: instruction issue, over the samples' steps. So a warp whose samples can no
+// longer collide leaves (clearOfEgo), and a tile none of whose samples can ends at once.
 // FAST: the fast arithmetic flavour and noise source (the default; the exact flavour
 // reproduces the oracle's per-sample results and serves parity tests). EGO (with FAST):
 // the ego's moves come from the instance's ego table of the plan (mppi_ego_table).
@@ -1129,17 +1398,38 @@ __global__ void __launch_bounds__(VERIFY_TILE, (verifyMinBlocks<NOPP, NTH>())) m
         const int T = D.cfg.T, H = D.cfg.H;
         const int plan = tile.aux;
         const uint32_t planBytes = (uint32_t)align16((size_t)NBP * T * 2 * 4);
-        unsigned* hist = (unsigned*)(smraw + offG + GRID_FLOATS * 4 + planBytes);
+        const uint32_t clearBytes = EGO ? (uint32_t)clearWords(H) * 4u : 0u;
+        float* sClear = (float*)(smraw + offG + GRID_FLOATS * 4 + planBytes);
+        unsigned* hist = (unsigned*)((unsigned char*)sClear + clearBytes);
         const int key = tile.inst * 2 + plan;
+        if constexpr (EGO)
+        {
+            // every sample starts from the same state: where it is clear of the ego over the
+            // whole horizon, no sample of the tile can fail
+            bool clear = !dbgTheta;
+            const ClearBlock<const float> cb(D.clear + (size_t)plan * clearWords(H), H);
+            clear = clear && *cb.out == 0.0f;
+            for (int o = 1; o <= NOPP; o++)
+                clear = clear && clearOfEgo(D.env, cb.xy, cb.all, H, 0, true, I.state.pos[2 * o], I.state.pos[2 * o + 1], I.state.vel[2 * o],
+                                            I.state.vel[2 * o + 1], D.env.maxSpeed[o], D.env.maxAccel[o]);
+            if (clear)
+            {
+                if constexpr (PQ)
+                    __syncthreads(); // every thread has read its ticket
+                continue;
+            }
+        }
         if (key != staged)
         {
             if (threadIdx.x == 0)
             {
-                mbar_expect_tx(bar, GRID_FLOATS * 4 + planBytes);
+                mbar_expect_tx(bar, GRID_FLOATS * 4 + planBytes + clearBytes);
                 if (!D.cfg.dbgNoStage)
                 {
                     bulk_g2s(sGrid, D.grids, GRID_FLOATS * 4, bar);
                     bulk_g2s(sPlan, plan == 0 ? D.dense : D.prevDense, planBytes, bar);
+                    if (EGO)
+                        bulk_g2s(sClear, D.clear + (size_t)plan * clearWords(H), clearBytes, bar);
                 }
             }
             copyEnv(sE, &D.env);
@@ -1158,6 +1448,15 @@ __global__ void __launch_bounds__(VERIFY_TILE, (verifyMinBlocks<NOPP, NTH>())) m
             }
             phase ^= 1u;
             staged = key;
+            if constexpr (EGO)
+            {
+                // from each group's own distances to those of it and the later ones
+                const ClearBlock<float> cb(sClear, H);
+                for (int j = threadIdx.x; j < H; j += blockDim.x)
+                    for (int g = clearGroups(H) - 2; g >= 0; g--)
+                        cb.rho[g * H + j] = fmaxf(cb.rho[g * H + j], cb.rho[(g + 1) * H + j]);
+                __syncthreads();
+            }
         }
         const EnvParams& E = *sE;
         const Track tr = trackIn(sGrid);
@@ -1214,6 +1513,22 @@ __global__ void __launch_bounds__(VERIFY_TILE, (verifyMinBlocks<NOPP, NTH>())) m
                 // the loop: see VERIFY_MIN_BLOCKS)
                 if (!__any_sync(0xffffffffu, active))
                     break;
+                if constexpr (EGO)
+                    if (t % CLEAR_EVERY == 0)
+                    {
+                        // or once none of them can fail any more (see clearOfEgo)
+                        // the group of the earliest branch that a sample has taken or can take
+                        const int tau = bs.predTheta == 0 || pt0 != 0 ? t : tOrigin - 1;
+                        const int gr = __reduce_min_sync(0xffffffffu, active ? (unsigned)tau : ~0u) / (unsigned)clearPer(H);
+                        const ClearBlock<const float> cb(sClear, H);
+                        bool clear = *cb.out == 0.0f;
+#pragma unroll
+                        for (int o = 1; o <= NOPP; o++)
+                            clear = clear && clearOfEgo(E, cb.xy, cb.rho + gr * H, H, t, active, st.pos[2 * o], st.pos[2 * o + 1], st.vel[2 * o],
+                                                        st.vel[2 * o + 1], E.maxSpeed[o], E.maxAccel[o]);
+                        if (clear)
+                            break;
+                    }
                 if (!active)
                     continue;
                 rng.begin_step((uint32_t)t);
@@ -1288,7 +1603,9 @@ size_t mppiRolloutSmem(int nopp, int nth, int T, int M, bool spl)
 
 size_t mppiVerifySmem(int nth, int T)
 {
-    return align16(16 + sizeof(EnvParams)) + GRID_FLOATS * 4 + ((((size_t)(nth + 1) * T * 2 * 4) + 15) & ~(size_t)15) + (size_t)T * 4;
+    // the clearance block of the longest verification horizon, T
+    return align16(16 + sizeof(EnvParams)) + GRID_FLOATS * 4 + ((((size_t)(nth + 1) * T * 2 * 4) + 15) & ~(size_t)15) +
+           ((size_t)T * (3 + CLEAR_GROUPS) + 4) * 4 + (size_t)T * 4;
 }
 
 template <int NOPP, int NTH, bool SPL> static cudaError_t launchRolloutS(const LaunchArgs& a, size_t smem)
@@ -1450,8 +1767,8 @@ cudaError_t launchMppiVerify(const LaunchArgs& a, int nopp, int nth, size_t smem
 cudaError_t launchEgoTable(cudaStream_t stream, int nopp, int nth, const MppiDev* insts, const MppiIn* in, int nInst, int plan, int maxH)
 {
     (void)nopp; // the ego's moves do not depend on the opponents
-    // blocks per instance: enough warps for the rows of the longest horizon of the batch
-    const dim3 grid(nInst, (unsigned)((egoRows(nth, maxH) + EGO_WARPS - 1) / EGO_WARPS));
+    // blocks per instance: enough for the rows of the longest horizon of the batch
+    const dim3 grid(nInst, (unsigned)((egoRows(nth, maxH) + EGO_CTA_ROWS - 1) / EGO_CTA_ROWS));
     switch (nth)
     {
     case 1: mppi_ego_table<1><<<grid, EGO_WARPS * 32, 0, stream>>>(insts, in, nInst, plan); break;
