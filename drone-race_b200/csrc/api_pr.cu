@@ -156,12 +156,23 @@ struct dr_prmppi_batch
     // draws no noise (its moves are then shared by the slots) and P is a multiple
     int slotsFor(int want) const
     {
-        if (envKind != 0 || want <= 1)
+        if (!egoShared() || want <= 1)
             return 1;
         for (auto* h : hs)
-            if (h->env.action_noise_level != 0.0f || h->env.pos_noise_level != 0.0f || h->env.speed_noise_level != 0.0f || h->P % want != 0)
+            if (h->P % want != 0)
                 return 1;
         return want;
+    }
+
+    // no controller's ego draws noise (strategic race)
+    bool egoShared() const
+    {
+        if (envKind != 0)
+            return false;
+        for (auto* h : hs)
+            if (h->env.action_noise_level != 0.0f || h->env.pos_noise_level != 0.0f || h->env.speed_noise_level != 0.0f)
+                return false;
+        return true;
     }
 
     LaunchArgs args(const Tile* tiles, int n, const PrIn* in) const
@@ -173,6 +184,7 @@ struct dr_prmppi_batch
         a.tiles = tiles;
         a.nTiles = n;
         a.prSlots = slotsFor(prSlots);
+        a.prShared = egoShared() ? 1 : 0;
         return a;
     }
 
@@ -193,7 +205,7 @@ struct dr_prmppi_batch
         CK(launchPrReduce(args(dWa, nWa, in)));
         if (profile)
             timer->mark("candidates", stream);
-        CK(envKind ? launchGatePrCandidates(args(nullptr, 0, in), nth, iMppi, n, maxT) : launchPrCandidates(args(nullptr, 0, in), nopp, nth, n, maxT, 0));
+        CK(envKind ? launchGatePrCandidates(args(nullptr, 0, in), nth, iMppi, n, maxT) : launchPrCandidates(args(nullptr, 0, in), nopp, nth, n, maxT, maxP));
         if (profile)
         {
             timer->mark("end", stream);
@@ -297,7 +309,7 @@ struct dr_prmppi_batch
         float* sums = mins + 3;
         CK(launchPrShardMerge(stream, dDesc, dIn, gathered, shardWords(), world, mins, sums));
         CK(launchPrShardApply(stream, dDesc, mins, sums));
-        CK(launchPrCandidates(args(nullptr, 0, dIn), nopp, nth, 1, maxT, 0));
+        CK(launchPrCandidates(args(nullptr, 0, dIn), nopp, nth, 1, maxT, maxP));
         int rc = copyResults();
         if (rc)
             return rc;
@@ -416,7 +428,7 @@ int buildPrBatch(dr_prmppi* const* hs, int n, cudaStream_t stream, bool ownStrea
     {
         dr_prmppi* h = hs[i];
         descs.push_back(h->desc);
-        const int spb = (h->envKind ? gatePrRolloutSamplesPerBlock() : prRolloutSamplesPerBlock()) / h->P;
+        const int spb = h->envKind ? gatePrRolloutSamplesPerBlock() / h->P : prRolloutSamplesPerTile(h->P);
         for (int nr = 0; nr < 2; nr++)
             for (int s0 = h->sLo; s0 < h->sHi; s0 += spb)
                 roll.push_back(Tile{i, s0, std::min(spb, h->sHi - s0), nr});
@@ -424,7 +436,7 @@ int buildPrBatch(dr_prmppi* const* hs, int n, cudaStream_t stream, bool ownStrea
             wa.push_back(Tile{i, w, 0, 0});
         b->maxT = std::max(b->maxT, h->T);
         b->maxP = std::max(b->maxP, h->P);
-        b->rollSmem = std::max(b->rollSmem, h->envKind ? gatePrRolloutSmem(h->T) : prRolloutSmem(h->T));
+        b->rollSmem = std::max(b->rollSmem, h->envKind ? gatePrRolloutSmem(h->T) : prRolloutSmem(h->T, h->P));
     }
     b->nRoll = (int)roll.size();
     b->nWa = (int)wa.size();

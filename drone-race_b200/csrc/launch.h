@@ -37,6 +37,9 @@ struct LaunchArgs
     int egoTable = 0;
     // PR-MPPI rollout: hypothesis slots per thread (1, 2, 4), sharing the ego's moves
     int prSlots = 1;
+    // PR-MPPI: 1 = no controller's ego draws noise, so that its moves are the same under every
+    // hypothesis and the kernels step it once for them
+    int prShared = 0;
 };
 
 inline int launchGrid(const LaunchArgs& a)
@@ -161,12 +164,12 @@ cudaError_t launchCp(cudaStream_t stream, const uint32_t* k, int n, uint32_t N, 
 cudaError_t launchTrackGrids(cudaStream_t stream, const double* q, int nTracks, float* out, float* lengths);
 
 bool prSupported(int nopp, int nth);
-int prRolloutSamplesPerBlock();
-size_t prRolloutSmem(int T);
+int prRolloutSamplesPerTile(int P);
+size_t prRolloutSmem(int T, int P);
 cudaError_t launchPrPrologue(const LaunchArgs& a, int nInst);
 cudaError_t launchPrRollout(const LaunchArgs& a, int nopp, int nth, size_t smem);
 cudaError_t launchPrReduce(const LaunchArgs& a);
-cudaError_t launchPrCandidates(const LaunchArgs& a, int nopp, int nth, int nInst, int maxP, size_t smem);
+cudaError_t launchPrCandidates(const LaunchArgs& a, int nopp, int nth, int nInst, int maxT, int maxP);
 cudaError_t launchPrNoise(const LaunchArgs& a, size_t n, float* out);
 
 } // namespace dr

@@ -339,4 +339,114 @@ __device__ __forceinline__ StepOut pairStep(unsigned mask, int role, int t, int 
     return r;
 }
 
+// ---- the opponent beside an ego that several hypotheses share -------------------------
+
+// One step of an ego that draws no noise, for the opponents of every hypothesis that meet it
+// (the ego's moves depend on its own action only): what their policies read before the step,
+// and the ego after it. Written by the ego's lane, read by its opponents' (shared memory,
+// [field][ego], so that the lanes of a field are neighbours).
+enum EgoField
+{
+    EF_S,     // before: arc length
+    EF_LAT,   //         lateral offset
+    EF_SDOT,  //         ds/dt
+    EF_ALONG, //         speed along the tangent
+    EF_PX,    // after: position
+    EF_PY,
+    EF_LAT1,  //        lateral offset
+    EF_LAPS1, //        laps (as an integer's bits)
+    EF_S1,    //        arc length
+    EGO_FIELDS
+};
+
+// The ego's step (egoStep, exact flavour) into its column of `row` (stride n).
+__device__ __forceinline__ void egoStepShared(const Track& tr, const EnvParams& E, float ego0, float ego1, DState<1>& s, float* row, int n)
+{
+    row[EF_S * n] = s.S[0];
+    row[EF_LAT * n] = s.lat[0];
+    const float v0 = s.vel[0], v1 = s.vel[1];
+    EgoRow r;
+    egoStep<false>(tr, E, ego0, ego1, s, r);
+    row[EF_SDOT * n] = r.sdot;
+    row[EF_ALONG * n] = v0 * r.tn0 + v1 * r.tn1;
+    row[EF_PX * n] = r.pos0;
+    row[EF_PY * n] = r.pos1;
+    row[EF_LAT1 * n] = r.lat;
+    row[EF_LAPS1 * n] = __int_as_float(r.laps);
+    row[EF_S1 * n] = r.S;
+}
+
+// The opponent's part of envStep<1, NTH, false, false, true, false> (no belief update, an
+// opponent's win ends the rollout) under hypothesis th, beside the ego's `row`; n0, n1 the
+// standard normals of its action noise.
+__device__ __forceinline__ StepOut oppStepShared(int th, const Track& tr, const EnvParams& E, DState<1>& s, const float* row, int n, float n0, float n1)
+{
+    const float prevS = s.S[0];
+    AgentGeo<1> g;
+    agentGeometry<1>(tr, E, s, g);
+    OppCommon c;
+    {
+        float pc0, pc1;
+        sampleAt2(tr.p, s.tp[0], pc0, pc1);
+        const float norm0 = -g.tn1[0], norm1 = g.tn0[0];
+        PairGeo q;
+        q.S[0] = row[EF_S * n];
+        q.S[1] = s.S[0];
+        q.lat[0] = row[EF_LAT * n];
+        q.lat[1] = s.lat[0];
+        q.sdot[0] = row[EF_SDOT * n];
+        q.sdot[1] = g.sdot[0];
+        q.egoLong = row[EF_ALONG * n];
+        q.tn0 = g.tn0[0];
+        q.tn1 = g.tn1[0];
+        q.kap = g.kap[0];
+        q.e_n = (s.pos[0] - pc0) * norm0 + (s.pos[1] - pc1) * norm1;
+        q.v_t = s.vel[0] * g.tn0[0] + s.vel[1] * g.tn1[0];
+        q.v_n = s.vel[0] * norm0 + s.vel[1] * norm1;
+        pairOppCommon(E, q, c);
+    }
+    float u0, u1;
+    oppAction<false>(1, th, E, c, u0, u1);
+    const float an = E.actionNoise[th][0];
+    if (an != 0.0f)
+    {
+        u0 += an * n0;
+        u1 += an * n1;
+    }
+    float sq = 0.0f;
+    sq += u0 * u0;
+    sq += u1 * u1;
+    float factor = 1.0f;
+    float maxSq = E.maxAccel[1] * E.maxAccel[1];
+    if (sq > maxSq)
+        factor = mdivsqrt<false>(E.maxAccel[1], sq);
+    u0 *= factor;
+    u1 *= factor;
+    s.pos[0] += E.dt * s.vel[0];
+    s.pos[1] += E.dt * s.vel[1];
+    s.S[0] += E.dt * g.sdot[0];
+    s.vel[0] += E.dt * u0;
+    s.vel[1] += E.dt * u1;
+    float sqSpd = sqNorm(s.vel[0], s.vel[1]);
+    if (sqSpd > E.maxSpeed[1] * E.maxSpeed[1])
+    {
+        float sc = mdivsqrt<false>(E.maxSpeed[1], sqSpd);
+        s.vel[0] *= sc;
+        s.vel[1] *= sc;
+    }
+    s.S[0] = projectOnTrack<false>(tr, E.trackLength, E.invTrackLength, s.pos[0], s.pos[1], s.S[0], s.lat[0], s.tp[0]);
+    if (s.S[0] < prevS - E.trackLength * 0.5f)
+        s.laps[0]++;
+    if (s.S[0] > prevS + E.trackLength * 0.5f)
+        s.laps[0]--;
+    StepOut r;
+    r.oppWon = s.laps[0] >= E.nWinLaps;
+    const float minSq = fminf(INFINITY, sqNorm(s.pos[0] - row[EF_PX * n], s.pos[1] - row[EF_PY * n]));
+    r.bdRaw = fminf(sqrtf(minSq) - E.droneRadius, E.trackWidth - fabsf(row[EF_LAT1 * n]));
+    r.winner = __float_as_int(row[EF_LAPS1 * n]) >= E.nWinLaps || fabsf(s.lat[0]) > E.trackWidth - E.droneRadius;
+    const float bdTerm = r.oppWon ? -1.0f : r.bdRaw;
+    r.term = bdTerm < E.droneRadius ? TERM_LOSE : r.winner ? TERM_WIN : TERM_NONE;
+    return r;
+}
+
 } // namespace dr

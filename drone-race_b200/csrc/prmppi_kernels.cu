@@ -21,6 +21,7 @@
 #include "common.cuh"
 #include "instance.cuh"
 #include "launch.h"
+#include "pair_model.cuh"
 
 namespace dr
 {
@@ -48,12 +49,14 @@ __host__ __device__ __forceinline__ size_t pa16(size_t x)
 }
 
 // Copies the host-filled part of EnvParams to shared memory and computes the
-// device-filled part; the caller's next __syncthreads publishes both.
+// device-filled part from there; all threads of the CTA, and the caller's next
+// __syncthreads publishes the terms.
 __device__ __forceinline__ void copyEnvP(EnvParams* dst, const EnvParams* src)
 {
     for (int i = threadIdx.x; i < ENV_HOST_WORDS; i += blockDim.x)
         ((float*)dst)[i] = ((const float*)src)[i];
-    envDeviceTerms(*dst, *src, threadIdx.x, blockDim.x);
+    __syncthreads();
+    envDeviceTerms(*dst, *dst, threadIdx.x, blockDim.x);
 }
 
 template <int NA> __device__ __forceinline__ void loadState(DState<NA>& st, const dr_sim_state& s)
@@ -356,6 +359,204 @@ __global__ void __launch_bounds__(PR_ROLL_TILE / HPT, prRollMinBlocks<NOPP>()) p
     }
 }
 
+// ---------------------------------------------------------------------------------------
+// rollout with one ego per sample (one opponent, an ego that draws no noise)
+// ---------------------------------------------------------------------------------------
+// A CTA of PRS_TILE threads: PrSplit::opp threads step an opponent each, one per (sample,
+// hypothesis), and the warps after them an ego each, one per sample, a step ahead of the
+// opponents (two rows of shared memory, the step's barrier in between).
+constexpr int PRS_TILE = 512;
+
+struct PrSplit
+{
+    int samples; // a tile's
+    int opp;     // threads that step opponents: whole warps
+};
+
+__host__ __device__ inline int prWarps(int threads)
+{
+    return (threads + 31) & ~31;
+}
+
+// the most samples whose opponents and egos fit PRS_TILE threads, and at most as many as the
+// tiles of the general kernel hold
+__host__ __device__ inline PrSplit prSplit(int P)
+{
+    int n = PR_ROLL_TILE / P;
+    while (prWarps(n * P) + prWarps(n) > PRS_TILE)
+        n--;
+    return PrSplit{n, prWarps(n * P)};
+}
+
+struct PrsSmem
+{
+    size_t env, grids, nom, rows, red, total;
+};
+
+__host__ __device__ inline PrsSmem prsLayout(int T, int P)
+{
+    auto a16 = [](size_t x) { return (x + 15) & ~(size_t)15; };
+    PrsSmem L;
+    const size_t n = prSplit(P).samples;
+    size_t off = 16;
+    L.env = off;
+    off = a16(off + sizeof(EnvParams));
+    L.grids = off;
+    off = a16(off + GRID_FLOATS * 4);
+    L.nom = off;
+    off = a16(off + (size_t)T * 2 * 4);
+    L.rows = off;
+    off = a16(off + 2 * EGO_FIELDS * n * 4);
+    L.red = off;
+    off = a16(off + n * P * 2 * 4);
+    L.total = off;
+    return L;
+}
+
+// What bounds it: instruction issue (73 % of the slots). Moving the ego was a good third of
+// the instructions of every hypothesis' rollout and is the same for all of a sample's; here it
+// is done once a sample. Its own warps step it beside the opponents instead of before them, so
+// the chain of a step is the opponent's alone; the barrier that the steps took already (it
+// keeps the warps on the same instructions) hands the rows over. 4 agents x 2 plans x 8
+// hypotheses x K 2048 x T 64, three mid-race states (B200, 1965 MHz): 0.49 / 0.35 / 0.47 ms
+// with an ego per hypothesis, 0.37 / 0.27 / 0.36 now; one agent of 2 x 9 x 65536 x 60 2.88 ->
+// 2.20 ms. Costs bit for bit the same.
+__global__ void __launch_bounds__(PRS_TILE, 2) pr_rollout_shared(const PrDev* __restrict__ insts, const PrIn* __restrict__ in, const Tile* __restrict__ tiles)
+{
+    extern __shared__ __align__(128) unsigned char smraw[];
+    const Tile tile = tiles[blockIdx.x];
+    const PrDev& D = insts[tile.inst];
+    const PrIn& I = in[tile.inst];
+    const int K = D.cfg.K, T = D.cfg.T, P = D.cfg.P;
+    const int robust = tile.aux;
+    const PrSplit split = prSplit(P);
+    const PrsSmem L = prsLayout(T, P);
+    uint64_t* bar = (uint64_t*)smraw;
+    EnvParams* sE = (EnvParams*)(smraw + L.env);
+    float* sGrid = (float*)(smraw + L.grids);
+    float* sNom = (float*)(smraw + L.nom);
+    float* rows = (float*)(smraw + L.rows);
+    float* red = (float*)(smraw + L.red);
+    const uint32_t nomBytes = (uint32_t)pa16((size_t)T * 2 * 4);
+    if (threadIdx.x == 0)
+    {
+        mbar_init(bar, 1);
+        mbar_expect_tx(bar, GRID_FLOATS * 4 + nomBytes);
+        bulk_g2s(sGrid, D.grids, GRID_FLOATS * 4, bar);
+        bulk_g2s(sNom, robust ? D.rob : D.nom, nomBytes, bar);
+    }
+    copyEnvP(sE, &D.env);
+    __syncthreads();
+    if (!__syncthreads_and(mbar_wait(bar, 0)))
+    {
+        if (threadIdx.x == 0)
+            atomicAdd(&D.stats[1], 1);
+        return;
+    }
+    const EnvParams& E = *sE;
+    const Track tr = trackIn(sGrid);
+    const int n = split.samples, rowWords = EGO_FIELDS * n;
+    const uint32_t k0 = D.cfg.k0, k1 = D.cfg.k1, step = I.step;
+    const bool ego = (int)threadIdx.x >= split.opp; // whole warps
+    const int a = ego ? 0 : 1;
+    DState<1> st;
+    st.pos[0] = I.state.pos[2 * a];
+    st.pos[1] = I.state.pos[2 * a + 1];
+    st.vel[0] = I.state.vel[2 * a];
+    st.vel[1] = I.state.vel[2 * a + 1];
+    st.S[0] = I.state.S[a];
+    st.lat[0] = I.state.lat_dist[a];
+    st.laps[0] = I.state.laps[a];
+    st.locate(E.trackLength);
+    if (ego)
+    {
+        const int sl = threadIdx.x - split.opp;
+        const bool valid = sl < n && sl < tile.count;
+        const uint32_t s = (uint32_t)(tile.s0 + sl);
+        // row t of the two is written while the opponents read row t - 1
+        for (int t = 0;; t++)
+        {
+            if (valid && t < T)
+            {
+                const U4 r = draw(k0, k1, s, (uint32_t)t, step, S_PR_EPS, 0);
+                const float ego0 = sNom[t * 2] + scaled_normal(D.cfg.sigma0, r.x);
+                const float ego1 = sNom[t * 2 + 1] + scaled_normal(D.cfg.sigma1, r.y);
+                egoStepShared(tr, E, ego0, ego1, st, rows + (t & 1) * rowWords + sl, n);
+            }
+            // one barrier a step: T of them, or fewer once the opponents are all done
+            if (t == T || !__syncthreads_or(0))
+                break;
+        }
+    }
+    else
+    {
+        const int sl = threadIdx.x / P, p = threadIdx.x % P;
+        const int s = tile.s0 + sl;
+        const bool valid = sl < n && sl < tile.count;
+        const int theta = D.thetas[p];
+        const uint32_t c1 = (((uint32_t)robust << 8) | (uint32_t)p) << 16;
+        const SafetyMargin margin = safetyMargin(E, D.cfg.collDistFactor);
+        float running = 0.0f, safe = -INFINITY, decay = 1.0f;
+        DState<2> last; // what the final cost reads
+        last.S[0] = I.state.S[0];
+        last.laps[0] = I.state.laps[0];
+        bool active = valid;
+        for (int t = 0; t < T; t++)
+        {
+            if (!__syncthreads_or(active))
+                break;
+            if (!active)
+                continue;
+            const float* row = rows + (t & 1) * rowWords + sl;
+            float n0 = 0.0f, n1 = 0.0f;
+            if (E.actionNoise[theta][0] != 0.0f)
+            {
+                const U4 r = draw(k0, k1, (uint32_t)s, c1 | (uint32_t)t, step, S_PR_ROLL_ENV, 0);
+                const float2 nn = normal_pair_ool(r.x, r.y);
+                n0 = nn.x;
+                n1 = nn.y;
+            }
+            const StepOut o = oppStepShared(theta, tr, E, st, row, n, n0, n1);
+            last.S[0] = row[EF_S1 * n];
+            last.laps[0] = __float_as_int(row[EF_LAPS1 * n]);
+            if (o.term != TERM_NONE)
+                active = false;
+            running += decay * prStateCost(o, E, D.cfg.boundaryThresholdFactor, D.cfg.boundaryCost, D.cfg.winCost, D.cfg.oppWinCost);
+            safe = fmaxf(safe, prSafetyCost(o, margin));
+            decay *= DECAY;
+        }
+        if (valid)
+        {
+            last.S[1] = st.S[0];
+            last.laps[1] = st.laps[0];
+            running += finalCost<1>(last, E, D.cfg.finalAdvWeight, D.cfg.finalOppAdvWeight);
+            float* out = robust ? D.costRob : D.costNom;
+            out[((size_t)p * K + s) * 2 + 0] = running;
+            out[((size_t)p * K + s) * 2 + 1] = safe;
+            red[(sl * P + p) * 2] = running;
+            red[(sl * P + p) * 2 + 1] = safe;
+        }
+    }
+    __syncthreads();
+    // PRMPPIcostAvgKernel (prmppi_kernels.cu:134-166)
+    for (int sl = threadIdx.x; sl < n && sl < tile.count; sl += blockDim.x)
+    {
+        const int s = tile.s0 + sl;
+        float avg = 0.0f, maxSafe = -INFINITY;
+        for (int q = 0; q < P; q++)
+        {
+            avg += red[(sl * P + q) * 2];
+            maxSafe = fmaxf(maxSafe, red[(sl * P + q) * 2 + 1]);
+        }
+        avg /= (float)P;
+        float full = avg + ((maxSafe > 0.0f) ? D.cfg.safetyWeight : 0.0f);
+        D.avg[((size_t)robust * K + s) * 2 + 0] = full;
+        D.avg[((size_t)robust * K + s) * 2 + 1] = maxSafe;
+        if (!isfinite(full))
+            atomicAdd(&D.stats[0], 1);
+    }
+}
+
 // block per (inst, which, t); tile.s0 = which * T + t
 __global__ void __launch_bounds__(PUB) pr_weighted(const PrDev* __restrict__ insts, const PrIn* __restrict__ in, const Tile* __restrict__ tiles)
 {
@@ -619,6 +820,43 @@ cudaError_t launchPrShardApply(cudaStream_t stream, const PrDev* insts, const fl
     return cudaGetLastError();
 }
 
+// The candidate choice (prmppi_controller.cu:236-256) and the safety decision (:264-275), by
+// thread 0, then the new plans; all threads of the instance's CTA, the candidates' costs
+// written and synchronised.
+__device__ __forceinline__ void prChoose(const PrDev& D, const float* sC1, const float* sC2, int T, int P, int* sChosen)
+{
+    if (threadIdx.x == 0)
+    {
+        float c1 = 0.0f, c2 = 0.0f;
+        for (int p = 0; p < P; ++p)
+        {
+            c1 += D.candFull[p];
+            c2 += D.candFull[P + p];
+        }
+        c1 /= (float)P;
+        c2 /= (float)P;
+        D.decision[0] = c2 < c1;          // resetNom
+        int chosen = (c1 <= c2) ? 0 : 1;
+        int useNom = 1;
+        for (int p = 0; p < P; p++)
+            if (D.candSafe[chosen * P + p] > 0.0f)
+            {
+                useNom = 0;
+                break;
+            }
+        D.decision[1] = useNom;
+        D.decision[2] = chosen;
+        *sChosen = chosen;
+    }
+    __syncthreads();
+    const float* ch = *sChosen ? sC2 : sC1;
+    for (int i = threadIdx.x; i < T * 2; i += blockDim.x)
+    {
+        D.nom[i] = ch[i];
+        D.rob[i] = D.robWork[i];
+    }
+}
+
 // one block per instance: threads (kind, cand, p), kind 0 = full cost, 1 = safety re-check
 template <int NOPP, int NTH>
 __global__ void __launch_bounds__(PRB) pr_candidates(const PrDev* __restrict__ insts, const PrIn* __restrict__ in, int nInst)
@@ -693,37 +931,134 @@ __global__ void __launch_bounds__(PRB) pr_candidates(const PrDev* __restrict__ i
             D.candSafe[tid] = safeCost;
     }
     __syncthreads();
-    // candidate choice (prmppi_controller.cu:236-256) and safety decision (:264-275)
+    prChoose(D, sC1, sC2, T, P, &sChosen);
+}
+
+// pr_candidates with the two candidates' egos shared by their opponents (one opponent, egos
+// that draw no noise): warps for the opponents (a lane per (kind, candidate, p)), as many that
+// draw their normals and one whose first two lanes move the egos, both a step ahead. What
+// bounds it is the chain of T steps of one warp, of whose instructions the ego and the draws
+// were about half: 0.23 -> 0.13 ms at T 64 (B200, 1965 MHz).
+constexpr int prCandWarps(int P)
+{
+    return (4 * P + 31) / 32;
+}
+
+__global__ void __launch_bounds__(9 * 32) pr_candidates_shared(const PrDev* __restrict__ insts, const PrIn* __restrict__ in, int nInst)
+{
+    extern __shared__ __align__(128) unsigned char smraw[];
+    __shared__ int sChosen;
+    __shared__ float rows[2][EGO_FIELDS * 2];
+    __shared__ float2 normals[2][4 * 32];
+    const int inst = blockIdx.x;
+    if (inst >= nInst)
+        return;
+    const PrDev& D = insts[inst];
+    const PrIn& I = in[inst];
+    const int T = D.cfg.T, P = D.cfg.P;
+    uint64_t* bar = (uint64_t*)smraw;
+    EnvParams* sE = (EnvParams*)(smraw + 16);
+    const size_t offG = pa16(16 + sizeof(EnvParams));
+    float* sGrid = (float*)(smraw + offG);
+    float* sC1 = (float*)(smraw + offG + GRID_FLOATS * 4);
+    const uint32_t cb = (uint32_t)pa16((size_t)T * 2 * 4);
+    float* sC2 = (float*)((unsigned char*)sC1 + cb);
     if (threadIdx.x == 0)
     {
-        float c1 = 0.0f, c2 = 0.0f;
-        for (int p = 0; p < P; ++p)
+        mbar_init(bar, 1);
+        mbar_expect_tx(bar, GRID_FLOATS * 4 + 2 * cb);
+        bulk_g2s(sGrid, D.grids, GRID_FLOATS * 4, bar);
+        bulk_g2s(sC1, D.cand1, cb, bar);
+        bulk_g2s(sC2, D.cand2, cb, bar);
+    }
+    copyEnvP(sE, &D.env);
+    __syncthreads();
+    if (!__syncthreads_and(mbar_wait(bar, 0)))
+    {
+        if (threadIdx.x == 0)
+            atomicAdd(&D.stats[1], 1);
+        return;
+    }
+    const EnvParams& E = *sE;
+    const Track tr = trackIn(sGrid);
+    const uint32_t k0 = D.cfg.k0, k1 = D.cfg.k1, step = I.step;
+    // the batch's widest controller sizes the block
+    const int group = ((int)blockDim.x / 32 - 1) / 2 * 32, role = threadIdx.x / group; // 0 opponents, 1 draws, 2 egos
+    const int task = threadIdx.x - role * group;
+    const int kind = task / (2 * P), tid = task % (2 * P);
+    const int second = role == 2 ? task : tid >= P;
+    const int p = tid >= P ? tid - P : tid;
+    const bool valid = role == 2 ? task < 2 : task < 4 * P;
+    const int a = role == 2 ? 0 : 1;
+    DState<1> st;
+    st.pos[0] = I.state.pos[2 * a];
+    st.pos[1] = I.state.pos[2 * a + 1];
+    st.vel[0] = I.state.vel[2 * a];
+    st.vel[1] = I.state.vel[2 * a + 1];
+    st.S[0] = I.state.S[a];
+    st.lat[0] = I.state.lat_dist[a];
+    st.laps[0] = I.state.laps[a];
+    st.locate(E.trackLength);
+    if (role != 0)
+    {
+        const float* nominal = second ? sC2 : sC1;
+        const bool noisy = role == 1 && valid && E.actionNoise[D.thetas[valid ? p : 0]][0] != 0.0f;
+        for (int t = 0;; t++)
         {
-            c1 += D.candFull[p];
-            c2 += D.candFull[P + p];
-        }
-        c1 /= (float)P;
-        c2 /= (float)P;
-        D.decision[0] = c2 < c1;          // resetNom
-        int chosen = (c1 <= c2) ? 0 : 1;
-        int useNom = 1;
-        for (int p = 0; p < P; p++)
-            if (D.candSafe[chosen * P + p] > 0.0f)
+            if (t < T)
             {
-                useNom = 0;
-                break;
+                if (role == 2 && valid)
+                    egoStepShared(tr, E, nominal[t * 2], nominal[t * 2 + 1], st, rows[t & 1] + second, 2);
+                else if (noisy)
+                {
+                    const U4 r = draw(k0, k1, (uint32_t)p, ((uint32_t)second << 16) | (uint32_t)t, step, kind ? S_PR_SAFE_ENV : S_PR_CAND_ENV, 0);
+                    normals[t & 1][task] = make_float2(normal_from_word(r.x), normal_from_word(r.y));
+                }
             }
-        D.decision[1] = useNom;
-        D.decision[2] = chosen;
-        sChosen = chosen;
+            if (t == T || !__syncthreads_or(0))
+                break;
+        }
+    }
+    else
+    {
+        const int theta = D.thetas[valid ? p : 0];
+        float cost = 0.0f, safeCost = -INFINITY, decay = 1.0f;
+        const SafetyMargin margin = safetyMargin(E, D.cfg.collDistFactor);
+        DState<2> last; // what the final cost reads
+        last.S[0] = I.state.S[0];
+        last.laps[0] = I.state.laps[0];
+        bool active = valid;
+        for (int t = 0; t < T; ++t)
+        {
+            if (!__syncthreads_or(active))
+                break;
+            if (!active)
+                continue;
+            const float* row = rows[t & 1] + second;
+            const float2 nn = normals[t & 1][task];
+            const StepOut o = oppStepShared(theta, tr, E, st, row, 2, nn.x, nn.y);
+            last.S[0] = row[EF_S1 * 2];
+            last.laps[0] = __float_as_int(row[EF_LAPS1 * 2]);
+            active = o.term == TERM_NONE;
+            cost += decay * prStateCost(o, E, D.cfg.boundaryThresholdFactor, D.cfg.boundaryCost, D.cfg.winCost, D.cfg.oppWinCost);
+            decay *= DECAY;
+            safeCost = fmaxf(safeCost, prSafetyCost(o, margin));
+        }
+        if (valid)
+        {
+            last.S[1] = st.S[0];
+            last.laps[1] = st.laps[0];
+            cost += finalCost<1>(last, E, D.cfg.finalAdvWeight, D.cfg.finalOppAdvWeight);
+            if (safeCost > 0.0f)
+                cost += D.cfg.safetyWeight;
+            if (kind == 0)
+                D.candFull[tid] = cost;
+            else
+                D.candSafe[tid] = safeCost;
+        }
     }
     __syncthreads();
-    const float* ch = sChosen ? sC2 : sC1;
-    for (int i = threadIdx.x; i < T * 2; i += blockDim.x)
-    {
-        D.nom[i] = ch[i];
-        D.rob[i] = D.robWork[i];
-    }
+    prChoose(D, sC1, sC2, T, P, &sChosen);
 }
 
 // perturbation of the next step, reference layout noise[T][K][2] (test hook)
@@ -746,14 +1081,15 @@ bool prSupported(int nopp, int nth)
     return key == 17 || key == 18 || key == 20 || key == 24 || key == 34;
 }
 
-int prRolloutSamplesPerBlock()
+int prRolloutSamplesPerTile(int P)
 {
-    return PR_ROLL_TILE;
+    return prSplit(P).samples;
 }
 
-size_t prRolloutSmem(int T)
+size_t prRolloutSmem(int T, int P)
 {
-    return prLayout(T).total;
+    const size_t a = prLayout(T).total, b = prsLayout(T, P).total;
+    return a > b ? a : b;
 }
 
 static size_t prCandSmem(int T)
@@ -776,9 +1112,18 @@ template <int NOPP, int NTH, int HPT> static cudaError_t prRollH(const LaunchArg
 }
 
 // a.prSlots hypothesis slots per thread (1, 2 or 4; the caller keeps it to 1 unless the
-// launch's egos draw no noise and P is a multiple of it)
+// launch's egos draw no noise and P is a multiple of it); with one, an ego per sample where
+// they draw none (a.prShared)
 template <int NOPP, int NTH> static cudaError_t prRollT(const LaunchArgs& a, size_t smem)
 {
+    if constexpr (NOPP == 1)
+        if (a.prShared && a.prSlots == 1)
+        {
+            auto k = pr_rollout_shared;
+            ensureSmem(k, smem);
+            k<<<a.nTiles, PRS_TILE, smem, a.stream>>>(a.pr, a.prIn, a.tiles);
+            return cudaGetLastError();
+        }
     switch (a.prSlots)
     {
     case 2: return prRollH<NOPP, NTH, 2>(a, smem);
@@ -787,8 +1132,17 @@ template <int NOPP, int NTH> static cudaError_t prRollT(const LaunchArgs& a, siz
     }
 }
 
-template <int NOPP, int NTH> static cudaError_t prCandT(const LaunchArgs& a, int nInst, int T)
+template <int NOPP, int NTH> static cudaError_t prCandT(const LaunchArgs& a, int nInst, int T, int P)
 {
+    if constexpr (NOPP == 1)
+        if (a.prShared)
+        {
+            auto k = pr_candidates_shared;
+            const size_t smem = prCandSmem(T);
+            ensureSmem(k, smem);
+            k<<<nInst, (2 * prCandWarps(P) + 1) * 32, smem, a.stream>>>(a.pr, a.prIn, nInst);
+            return cudaGetLastError();
+        }
     auto k = pr_candidates<NOPP, NTH>;
     size_t smem = prCandSmem(T);
     ensureSmem(k, smem);
@@ -820,9 +1174,9 @@ cudaError_t launchPrReduce(const LaunchArgs& a)
     return cudaGetLastError();
 }
 
-cudaError_t launchPrCandidates(const LaunchArgs& a, int nopp, int nth, int nInst, int maxT, size_t)
+cudaError_t launchPrCandidates(const LaunchArgs& a, int nopp, int nth, int nInst, int maxT, int maxP)
 {
-#define CALL(P_, Q_) prCandT<P_, Q_>(a, nInst, maxT)
+#define CALL(P_, Q_) prCandT<P_, Q_>(a, nInst, maxT, maxP)
     DR_PR_DISPATCH(nopp, nth, CALL)
 #undef CALL
 }
