@@ -273,6 +273,14 @@ struct dr_mppi_batch
         return true;
     }
 
+    int maxSamples() const
+    {
+        int k = 0;
+        for (auto* h : hs)
+            k = std::max(k, h->K);
+        return k;
+    }
+
     cudaError_t launchEgo(cudaStream_t s, const MppiIn* in, int plans) const
     {
         if (!egoTable())
@@ -413,7 +421,7 @@ struct dr_mppi_batch
             // side verification's pending CTAs, and wait in the kernel for its results
             LaunchArgs ua = args(dUpd, nUpd, in);
             ua.pdl = pdl;
-            CK(launchMppiUpdate(ua, nth));
+            CK(launchMppiUpdate(ua, nth, maxSamples()));
         }
         if (nGrad > 0)
         {
@@ -838,6 +846,8 @@ int buildMppiBatch(dr_mppi* const* hs, int n, cudaStream_t stream, bool ownStrea
         });
     };
     byWork(roll, false);
+    // the update's blocks go over their controller's samples: most samples first
+    std::stable_sort(upd.begin(), upd.end(), [&](const Tile& x, const Tile& y) { return hs[x.inst]->K > hs[y.inst]->K; });
     byWork(ver, true);
     byWork(verOld, true);
     // tile table: new-plan tiles first, then previous-plan tiles
@@ -1722,7 +1732,7 @@ int dr_mppi_debug_update(dr_mppi* h, const float* belief, const float* costs_tru
     CK(cudaMemcpyAsync(h->desc.costsTrue, costs_true, nk * 4, cudaMemcpyHostToDevice, h->stream));
     CK(cudaMemcpyAsync(h->desc.binfo, info.data(), nk * 4, cudaMemcpyHostToDevice, h->stream));
     CK(launchMppiAggregate(b->args(nullptr, 0, b->dIn), h->nth, h->K));
-    CK(launchMppiUpdate(b->args(b->dUpd, b->nUpd, b->dIn), h->nth));
+    CK(launchMppiUpdate(b->args(b->dUpd, b->nUpd, b->dIn), h->nth, b->maxSamples()));
     if (dense_nominal)
         CK(cudaMemcpyAsync(dense_nominal, h->desc.dense, (size_t)h->nbp * h->T * 2 * 4, cudaMemcpyDeviceToHost, h->stream));
     if (min_costs)

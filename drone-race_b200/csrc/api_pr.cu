@@ -175,6 +175,14 @@ struct dr_prmppi_batch
         return true;
     }
 
+    int maxSamples() const
+    {
+        int k = 0;
+        for (auto* h : hs)
+            k = std::max(k, h->K);
+        return k;
+    }
+
     LaunchArgs args(const Tile* tiles, int n, const PrIn* in) const
     {
         LaunchArgs a;
@@ -202,7 +210,7 @@ struct dr_prmppi_batch
         CK(envKind ? launchGatePrRollout(args(dRoll, nRoll, in), nth, iMppi, rollSmem) : launchPrRollout(args(dRoll, nRoll, in), nopp, nth, rollSmem));
         if (profile)
             timer->mark("weighted", stream);
-        CK(launchPrReduce(args(dWa, nWa, in)));
+        CK(launchPrReduce(args(dWa, nWa, in), maxSamples()));
         if (profile)
             timer->mark("candidates", stream);
         CK(envKind ? launchGatePrCandidates(args(nullptr, 0, in), nth, iMppi, n, maxT) : launchPrCandidates(args(nullptr, 0, in), nopp, nth, n, maxT, maxP));
@@ -432,7 +440,7 @@ int buildPrBatch(dr_prmppi* const* hs, int n, cudaStream_t stream, bool ownStrea
         for (int nr = 0; nr < 2; nr++)
             for (int s0 = h->sLo; s0 < h->sHi; s0 += spb)
                 roll.push_back(Tile{i, s0, std::min(spb, h->sHi - s0), nr});
-        for (int w = 0; w < 3 * h->T; w++)
+        for (int w = 0; w < h->T; w++) // a step's three averages
             wa.push_back(Tile{i, w, 0, 0});
         b->maxT = std::max(b->maxT, h->T);
         b->maxP = std::max(b->maxP, h->P);

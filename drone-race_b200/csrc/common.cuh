@@ -113,6 +113,27 @@ inline cudaError_t launchMaybePdl(bool pdl, void (*k)(KArgs...), dim3 grid, dim3
     return cudaLaunchKernelEx(&cfg, k, args...);
 }
 
+// launchMaybePdl with clusters of `c` CTAs along x.
+template <typename... KArgs, typename... Args>
+inline cudaError_t launchCluster(bool pdl, int c, void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)c;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = pdl ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, k, args...);
+}
+
 // The tile a CTA works on in iteration `iter` of its tile loop. A static launch (no queue)
 // has one CTA per tile: its own, once. A persistent launch takes the next ticket of the
 // device work queue (tiles in table order, so the table lists the longest tiles first);

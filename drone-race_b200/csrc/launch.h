@@ -68,7 +68,8 @@ size_t mppiRolloutSmem(int nopp, int nth, int T, int M, bool spl);
 size_t mppiVerifySmem(int nth, int T);
 cudaError_t launchMppiPrologue(const LaunchArgs& a, int nInst, size_t smem);
 cudaError_t launchMppiRollout(const LaunchArgs& a, int nopp, int nth, bool spl, size_t smem);
-cudaError_t launchMppiUpdate(const LaunchArgs& a, int nth);
+// maxK: the most samples of a controller of the launch
+cudaError_t launchMppiUpdate(const LaunchArgs& a, int nth, int maxK);
 cudaError_t launchMppiAggregate(const LaunchArgs& a, int nth, int K);
 // sample-sharded update phases (one controller's samples split across processes)
 cudaError_t launchShardLocal(const LaunchArgs& a, int nth, float* partial);
@@ -168,7 +169,8 @@ int prRolloutSamplesPerTile(int P);
 size_t prRolloutSmem(int T, int P);
 cudaError_t launchPrPrologue(const LaunchArgs& a, int nInst);
 cudaError_t launchPrRollout(const LaunchArgs& a, int nopp, int nth, size_t smem);
-cudaError_t launchPrReduce(const LaunchArgs& a);
+// maxK: the most samples of a controller of the launch
+cudaError_t launchPrReduce(const LaunchArgs& a, int maxK);
 cudaError_t launchPrCandidates(const LaunchArgs& a, int nopp, int nth, int nInst, int maxT, int maxP);
 cudaError_t launchPrNoise(const LaunchArgs& a, size_t n, float* out);
 

@@ -9,7 +9,7 @@
 //                  (PRMPPIfullRolloutKernel, :55-130); the hypotheses of a sample sit in
 //                  neighbouring threads, so the per-sample average over p and the safety
 //                  indicator (PRMPPIcostAvgKernel, :134-166) are done in the epilogue.
-//   pr_weighted    per (which, t): minimum of the averaged cost (PRMPPIcomputeMinCosts-
+//   pr_weighted    per t, the three averages: minimum of the averaged cost (PRMPPIcomputeMinCosts-
 //                  Kernel, :169-199), exponential weights and the weighted average of the
 //                  absolute perturbed controls (PRMPPIWeightedAverageKernel, :204-282),
 //                  with the perturbation regenerated and the sums in the reference's order.
@@ -18,10 +18,14 @@
 //                  re-check of the one that will be chosen (PRMPPIcomputeSafeCostKernel,
 //                  :350-393); then the choice itself (prmppi_controller.cu:232-304) so
 //                  that the host needs one synchronisation per step.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 #include "instance.cuh"
 #include "launch.h"
 #include "pair_model.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace dr
 {
@@ -557,64 +561,172 @@ __global__ void __launch_bounds__(PRS_TILE, 2) pr_rollout_shared(const PrDev* __
     }
 }
 
-// block per (inst, which, t); tile.s0 = which * T + t
+// The three weighted averages of a step t (tile.s0 = t), one cluster of C CTAs: which 0:
+// nominal + full cost; 1: robust + full cost; 2: robust + safety cost. They share the samples'
+// perturbations of the step, so each is drawn once for the three. The sums keep the
+// reference's order: lane l of its 256 adds samples l, l + 256, ... one after the other, then
+// the lanes are added in a tree; each CTA takes 256 / C lanes, computes C samples of a lane
+// side by side and adds their terms in order from shared memory (as mppi_update does, whose
+// comment says why). C = 1: a thread is a lane.
+template <int C>
 __global__ void __launch_bounds__(PUB) pr_weighted(const PrDev* __restrict__ insts, const PrIn* __restrict__ in, const Tile* __restrict__ tiles)
 {
-    __shared__ float sA[PUB], sB[PUB], sC[PUB];
-    __shared__ float sMin[PUB / 32];
-    const Tile tile = tiles[blockIdx.x];
+    constexpr int W = PUB / C; // lanes of this CTA
+    constexpr int R = 2;       // terms a thread computes between two barriers (C > 1)
+    __shared__ float sSum[9][PUB]; // per average: weighted controls and weights
+    __shared__ float sMin[3][PUB / 32];
+    __shared__ float sMinAll[3][C];
+    __shared__ float sTerm[5][C > 1 ? 2 * R * PUB : 1]; // the three weights and the perturbation of C R samples a lane, twice
+    if constexpr (C > 1)
+        cg::this_cluster().barrier_arrive(); // this CTA runs: its shared memory may be written
+    const Tile tile = tiles[blockIdx.x / C];
     const PrDev& D = insts[tile.inst];
     const PrIn& I = in[tile.inst];
-    const int K = D.cfg.K, T = D.cfg.T;
-    const int which = tile.s0 / T, t = tile.s0 % T;
+    const int K = D.cfg.K, t = tile.s0;
     const int tid = threadIdx.x;
-    // which 0: nominal + full cost; 1: robust + full cost; 2: robust + safety cost
-    const float* arr = D.avg + (size_t)(which == 0 ? 0 : K) * 2 + (which == 2 ? 1 : 0);
-    const float* nominal = which == 0 ? D.nom : D.rob;
-    float mn = INFINITY;
-    for (int s = tid; s < K; s += PUB)
-        mn = fminf(mn, arr[(size_t)s * 2]);
-    mn = warp_min(mn);
-    if ((tid & 31) == 0)
-        sMin[tid >> 5] = mn;
-    __syncthreads();
-    float minCost = sMin[0];
-#pragma unroll
-    for (int w = 1; w < PUB / 32; w++)
-        minCost = fminf(minCost, sMin[w]);
-    const float invTemp = I.lambda[which];
-    const float nom0 = nominal[t * 2], nom1 = nominal[t * 2 + 1];
-    const uint32_t k0 = D.cfg.k0, k1 = D.cfg.k1, step = I.step;
-    float num0 = 0.0f, num1 = 0.0f, den = 0.0f;
-    for (int s = tid; s < K; s += PUB)
+    const int rank = C > 1 ? blockIdx.x % C : 0;
+    const int first = (tid / W) * PUB + rank * W + tid % W; // this thread's first sample; then every C PUB
+    const float2* nomAvg = (const float2*)D.avg; // (full, safety) cost of a sample: nominal, then robust
+    const float2* robAvg = nomAvg + K;
+    float mn[3] = {INFINITY, INFINITY, INFINITY};
+    for (int s = first; s < K; s += C * PUB)
     {
-        float cost = arr[(size_t)s * 2];
-        float w = expf(-(cost - minCost) / invTemp);
-        U4 r = draw(k0, k1, (uint32_t)s, (uint32_t)t, step, S_PR_EPS, 0);
-        float u0 = nom0 + scaled_normal(D.cfg.sigma0, r.x);
-        float u1 = nom1 + scaled_normal(D.cfg.sigma1, r.y);
-        num0 += w * u0;
-        num1 += w * u1;
-        den += w;
+        const float2 r = robAvg[s];
+        mn[0] = fminf(mn[0], nomAvg[s].x);
+        mn[1] = fminf(mn[1], r.x);
+        mn[2] = fminf(mn[2], r.y);
     }
-    sA[tid] = num0;
-    sB[tid] = num1;
-    sC[tid] = den;
+    float minCost[3];
+#pragma unroll
+    for (int w = 0; w < 3; w++)
+    {
+        mn[w] = warp_min(mn[w]);
+        if ((tid & 31) == 0)
+            sMin[w][tid >> 5] = mn[w];
+    }
     __syncthreads();
+#pragma unroll
+    for (int w = 0; w < 3; w++)
+    {
+        minCost[w] = sMin[w][0];
+#pragma unroll
+        for (int i = 1; i < PUB / 32; i++)
+            minCost[w] = fminf(minCost[w], sMin[w][i]);
+    }
+    if constexpr (C > 1)
+    {
+        // every CTA of the cluster gets every CTA's minima
+        cg::cluster_group cluster = cg::this_cluster();
+        cluster.barrier_wait();
+        if (tid < C)
+#pragma unroll
+            for (int w = 0; w < 3; w++)
+                cluster.map_shared_rank(&sMinAll[w][0], tid)[rank] = minCost[w];
+        cluster.sync();
+#pragma unroll
+        for (int w = 0; w < 3; w++)
+#pragma unroll
+            for (int q = 0; q < C; q++)
+                minCost[w] = fminf(minCost[w], sMinAll[w][q]);
+    }
+    float invTemp[3], nom0[3], nom1[3];
+#pragma unroll
+    for (int w = 0; w < 3; w++)
+    {
+        invTemp[w] = I.lambda[w];
+        const float* nominal = w == 0 ? D.nom : D.rob;
+        nom0[w] = nominal[t * 2];
+        nom1[w] = nominal[t * 2 + 1];
+    }
+    const uint32_t k0 = D.cfg.k0, k1 = D.cfg.k1, step = I.step;
+    float sum[9] = {};
+    struct Term
+    {
+        float w[3], e0, e1;
+    };
+    auto term = [&](int s) {
+        Term v;
+        const float2 r = robAvg[s];
+        const float cost[3] = {nomAvg[s].x, r.x, r.y};
+#pragma unroll
+        for (int w = 0; w < 3; w++)
+            v.w[w] = expf(-(cost[w] - minCost[w]) / invTemp[w]);
+        const U4 d = draw(k0, k1, (uint32_t)s, (uint32_t)t, step, S_PR_EPS, 0);
+        v.e0 = scaled_normal(D.cfg.sigma0, d.x);
+        v.e1 = scaled_normal(D.cfg.sigma1, d.y);
+        return v;
+    };
+    auto add = [&](const Term& v) {
+#pragma unroll
+        for (int w = 0; w < 3; w++)
+        {
+            const float u0 = nom0[w] + v.e0, u1 = nom1[w] + v.e1;
+            sum[3 * w] += v.w[w] * u0;
+            sum[3 * w + 1] += v.w[w] * u1;
+            sum[3 * w + 2] += v.w[w];
+        }
+    };
+    if constexpr (C == 1)
+    {
+        for (int s = tid; s < K; s += PUB)
+            add(term(s));
+#pragma unroll
+        for (int i = 0; i < 9; i++)
+            sSum[i][tid] = sum[i];
+        __syncthreads();
+    }
+    else
+    {
+        int buf = 0;
+        for (int s0 = 0; s0 < K; s0 += R * C * PUB, buf ^= R * PUB)
+        {
+#pragma unroll
+            for (int r = 0; r < R; r++)
+            {
+                const int s = s0 + r * C * PUB + first, at = buf + r * PUB + tid; // [(r, sample of the lane)][lane]
+                if (s < K)
+                {
+                    const Term v = term(s);
+                    sTerm[0][at] = v.w[0];
+                    sTerm[1][at] = v.w[1];
+                    sTerm[2][at] = v.w[2];
+                    sTerm[3][at] = v.e0;
+                    sTerm[4][at] = v.e1;
+                }
+            }
+            __syncthreads();
+            if (tid < W)
+#pragma unroll 4
+                for (int i = 0; i < R * C; i++)
+                    if (s0 + i * PUB + rank * W + tid < K)
+                    {
+                        const int at = buf + i * W + tid;
+                        add(Term{{sTerm[0][at], sTerm[1][at], sTerm[2][at]}, sTerm[3][at], sTerm[4][at]});
+                    }
+        }
+        // all lanes' sums to the cluster's first CTA, which goes on alone
+        cg::cluster_group cluster = cg::this_cluster();
+        if (tid < W)
+#pragma unroll
+            for (int i = 0; i < 9; i++)
+                cluster.map_shared_rank(&sSum[i][0], 0)[rank * W + tid] = sum[i];
+        cluster.sync();
+        if (rank != 0)
+            return;
+    }
 #pragma unroll
     for (int stride = PUB / 2; stride >= 32; stride >>= 1)
     {
         if (tid < stride)
-        {
-            sA[tid] += sA[tid + stride];
-            sB[tid] += sB[tid + stride];
-            sC[tid] += sC[tid + stride];
-        }
+#pragma unroll
+            for (int i = 0; i < 9; i++)
+                sSum[i][tid] += sSum[i][tid + stride];
         __syncthreads();
     }
-    if (tid < 32)
+    const int which = tid >> 5, l = tid & 31; // a warp per average
+    if (which < 3)
     {
-        float a0 = sA[tid], a1 = sB[tid], dd = sC[tid];
+        float a0 = sSum[3 * which][l], a1 = sSum[3 * which + 1][l], dd = sSum[3 * which + 2][l];
 #pragma unroll
         for (int stride = 16; stride > 0; stride >>= 1)
         {
@@ -622,15 +734,16 @@ __global__ void __launch_bounds__(PUB) pr_weighted(const PrDev* __restrict__ ins
             a1 += __shfl_down_sync(0xffffffffu, a1, stride);
             dd += __shfl_down_sync(0xffffffffu, dd, stride);
         }
-        if (tid == 0)
+        if (l == 0)
         {
             float* out = which == 0 ? D.cand1 : (which == 1 ? D.cand2 : D.robWork);
-            out[t * 2] = (dd > 1e-30f) ? a0 / dd : nom0;
-            out[t * 2 + 1] = (dd > 1e-30f) ? a1 / dd : nom1;
+            const float* nominal = which == 0 ? D.nom : D.rob;
+            out[t * 2] = (dd > 1e-30f) ? a0 / dd : nominal[t * 2];
+            out[t * 2 + 1] = (dd > 1e-30f) ? a1 / dd : nominal[t * 2 + 1];
             if (t == 0)
             {
                 D.nu[which] = dd;
-                D.minCosts[which] = minCost;
+                D.minCosts[which] = which == 0 ? minCost[0] : which == 1 ? minCost[1] : minCost[2];
             }
         }
     }
@@ -1168,10 +1281,22 @@ cudaError_t launchPrRollout(const LaunchArgs& a, int nopp, int nth, size_t smem)
 #undef CALL
 }
 
-cudaError_t launchPrReduce(const LaunchArgs& a)
+// CTAs per step of the weighted averages: as mppi_update's clusters (updateCluster), as many as
+// it takes to give every SM two, while a thread still has four samples (three averages each).
+// One agent of K 65536, T 60 (B200, 1965 MHz): 0.278 ms with a block per (average, step), 0.088
+// with eight CTAs a step; four agents of K 2048, T 64: 0.030 -> 0.020 with two.
+cudaError_t launchPrReduce(const LaunchArgs& a, int maxK)
 {
-    pr_weighted<<<a.nTiles, PUB, 0, a.stream>>>(a.pr, a.prIn, a.tiles);
-    return cudaGetLastError();
+    int c = 1;
+    while (c < 8 && a.nTiles * c < 296 && maxK >= 2 * c * PUB * 4)
+        c *= 2;
+    switch (c)
+    {
+    case 8: return launchCluster(false, 8, pr_weighted<8>, dim3(a.nTiles * 8), dim3(PUB), 0, a.stream, a.pr, a.prIn, a.tiles);
+    case 4: return launchCluster(false, 4, pr_weighted<4>, dim3(a.nTiles * 4), dim3(PUB), 0, a.stream, a.pr, a.prIn, a.tiles);
+    case 2: return launchCluster(false, 2, pr_weighted<2>, dim3(a.nTiles * 2), dim3(PUB), 0, a.stream, a.pr, a.prIn, a.tiles);
+    default: pr_weighted<1><<<a.nTiles, PUB, 0, a.stream>>>(a.pr, a.prIn, a.tiles); return cudaGetLastError();
+    }
 }
 
 cudaError_t launchPrCandidates(const LaunchArgs& a, int nopp, int nth, int nInst, int maxT, int maxP)
