@@ -110,18 +110,18 @@ __device__ __forceinline__ float acklam_tail(float q)
     return __fdiv_rn(num, den);
 }
 
+// Both tails in one branch (the upper one is the lower one of 1 - u with the sign changed): one
+// lane in twenty takes it, so a warp nearly always does, once where two branches were taken
+// (B200, 1965 MHz: the PR-MPPI rollout of 4 x 2 x 8 x 2048 x 64 0.37 -> 0.35 ms, the gate
+// race's of 4 x 2 x 4096 x 64 0.31 -> 0.28 beside the verification).
 __device__ __forceinline__ float normal_from_uniform(float u)
 {
     const float plow = 0.02425f;
-    if (u < plow)
+    if (u < plow || u > __fsub_rn(1.0f, plow))
     {
-        float q = __fsqrt_rn(__fmul_rn(-2.0f, series_logf(u)));
-        return acklam_tail(q);
-    }
-    if (u > __fsub_rn(1.0f, plow))
-    {
-        float q = __fsqrt_rn(__fmul_rn(-2.0f, series_logf(__fsub_rn(1.0f, u))));
-        return -acklam_tail(q);
+        const float v = u < plow ? u : __fsub_rn(1.0f, u);
+        const float x = acklam_tail(__fsqrt_rn(__fmul_rn(-2.0f, series_logf(v))));
+        return u < plow ? x : -x;
     }
     float q = __fsub_rn(u, 0.5f);
     float r = __fmul_rn(q, q);
