@@ -114,8 +114,9 @@ __device__ __forceinline__ void pairOppCommon(const EnvParams& E, const PairGeo&
 // Everything the two lanes return is the same on both, except `s`. Hypotheses are evaluated
 // two at a time, an even one on the ego's lane and the next on the opponent's; a round whose
 // hypotheses all repeat an earlier one's action (EnvParams::dupAll / dupNoBlock) is skipped,
-// and a committed sample evaluates the true hypothesis only.
-template <int NTH>
+// and a committed sample evaluates the true hypothesis only. LOSE: an opponent's win ends the
+// rollout as a loss (loseOnOppWin); NOISE: the environment's own noise, where it is on, is drawn.
+template <int NTH, bool LOSE = true, bool NOISE = true>
 __device__ __forceinline__ StepOut pairStep(unsigned mask, int role, int t, int trueTheta, const Track& tr, const EnvParams& E, float ctl0, float ctl1,
                                             float opp0, float opp1, DState<1>& s, BState<NTH>& bs, bool& branched, float minConf, const PairNoise& noise)
 {
@@ -214,7 +215,7 @@ __device__ __forceinline__ StepOut pairStep(unsigned mask, int role, int t, int 
             factor = mdivsqrt<false>(maxAccel, sq);
         act0 *= factor;
         act1 *= factor;
-        if (E.actionNoiseLevel != 0.0f)
+        if (NOISE && E.actionNoiseLevel != 0.0f)
         {
             act0 += noise.at(jn + 2 * role) * E.actionNoiseLevel;
             act1 += noise.at(jn + 2 * role + 1) * E.actionNoiseLevel;
@@ -237,7 +238,7 @@ __device__ __forceinline__ StepOut pairStep(unsigned mask, int role, int t, int 
         }
     }
     // 7. state noise: per agent and axis a position normal, then a speed normal
-    if (E.posNoise != 0.0f || E.speedNoise != 0.0f)
+    if (NOISE && (E.posNoise != 0.0f || E.speedNoise != 0.0f))
     {
         const int per = (E.posNoise != 0.0f ? 1 : 0) + (E.speedNoise != 0.0f ? 1 : 0);
         int j = jn + role * 2 * per;
@@ -334,8 +335,8 @@ __device__ __forceinline__ StepOut pairStep(unsigned mask, int role, int t, int 
     const float minSq = fminf(INFINITY, sqNorm(po0 - pe0, po1 - pe1));
     r.bdRaw = fminf(sqrtf(minSq) - E.droneRadius, E.trackWidth - fabsf(le));
     r.winner = he >= E.nWinLaps || fabsf(lo) > E.trackWidth - E.droneRadius;
-    const float bdTerm = r.oppWon ? -1.0f : r.bdRaw;
-    r.term = bdTerm < E.droneRadius ? TERM_LOSE : r.winner ? TERM_WIN : TERM_NONE;
+    const float bdTerm = (LOSE && r.oppWon) ? -1.0f : r.bdRaw;
+    r.term = bdTerm < E.droneRadius ? TERM_LOSE : r.winner ? TERM_WIN : !LOSE && r.oppWon ? TERM_OPP_WIN : TERM_NONE;
     return r;
 }
 
