@@ -58,6 +58,7 @@ struct dr_mppi
                env.speed_noise_level == 0.0f;
     }
     DevScratch predBuf; // dr_mppi_predict's inputs and outputs on the device
+    PinnedScratch hPred; // and in pinned host memory
     Arena arena;
     MppiDev desc{};
     unsigned char* hRes = nullptr; // pinned copy of the result block
@@ -1226,6 +1227,7 @@ int dr_mppi_destroy(dr_mppi* h)
     cudaFree(h->dGradIn);
     cudaFree(h->dGradJobs);
     h->predBuf.release();
+    h->hPred.release();
     if (h->desc.cpFull)
         releaseCpTable(h->device, (uint32_t)h->V, h->cpBeta);
     h->arena.release();
@@ -1853,22 +1855,27 @@ int dr_mppi_predict(dr_mppi* h, const dr_sim_state* state, const float* belief, 
                  oAct = oPos + a256(nPos * 4), oRec = oAct + a256(nAct * 4), oCost = oRec + a256(nRec * 4), total = oCost + a256((size_t)nth * 4);
     CK(h->predBuf.reserve(total));
     unsigned char* base = (unsigned char*)h->predBuf.p;
+    // inputs and outputs in one copy each, through pinned memory
+    CK(h->hPred.reserve(total));
+    unsigned char* host = (unsigned char*)h->hPred.p;
     // the record carries the pending warm-start shift that the engine's h_nominal holds
     MppiIn in = h->input(*state, belief);
     float bel[DR_MAX_THETA] = {};
     for (int i = 0; i < nth; i++)
         bel[i] = belief[i];
-    CK(cudaMemcpyAsync(base + oIn, &in, sizeof(MppiIn), cudaMemcpyHostToDevice, h->stream));
-    CK(cudaMemcpyAsync(base + oSt, state, sizeof(dr_sim_state), cudaMemcpyHostToDevice, h->stream));
-    CK(cudaMemcpyAsync(base + oBel, bel, sizeof(bel), cudaMemcpyHostToDevice, h->stream));
+    std::memcpy(host + oIn, &in, sizeof(MppiIn));
+    std::memcpy(host + oSt, state, sizeof(dr_sim_state));
+    std::memcpy(host + oBel, bel, sizeof(bel));
+    CK(cudaMemcpyAsync(base, host, oPos, cudaMemcpyHostToDevice, h->stream));
     PredictOut out{(float*)(base + oPos), (float*)(base + oAct), (int*)(base + oRec), (float*)(base + oCost), T};
     CK(launchMppiPredict(h->stream, h->nopp, nth, h->self->dDesc, (const MppiIn*)(base + oIn), (const dr_sim_state*)(base + oSt),
                          (const float*)(base + oBel), DR_MAX_THETA, out, 1));
-    CK(cudaMemcpyAsync(positions, base + oPos, nPos * 4, cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaMemcpyAsync(actions, base + oAct, nAct * 4, cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaMemcpyAsync(records, base + oRec, nRec * 4, cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaMemcpyAsync(costs, base + oCost, (size_t)nth * 4, cudaMemcpyDeviceToHost, h->stream));
+    CK(cudaMemcpyAsync(host + oPos, base + oPos, total - oPos, cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
+    std::memcpy(positions, host + oPos, nPos * 4);
+    std::memcpy(actions, host + oAct, nAct * 4);
+    std::memcpy(records, host + oRec, nRec * 4);
+    std::memcpy(costs, host + oCost, (size_t)nth * 4);
     return DR_OK;
 }
 

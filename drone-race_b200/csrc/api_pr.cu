@@ -1039,19 +1039,26 @@ extern "C" int dr_env_step(const dr_env_config* env, int true_theta, const float
         return fail(DR_ERR_UNSUPPORTED, "(n_opp, n_theta) combination not compiled in");
     int dev = 0;
     CK(cudaGetDevice(&dev));
-    std::vector<float> g = packGrids(*env);
+    // one step: a scan of the projection windows costs the device less than their
+    // certificates cost the host (0.46 -> 0.06 ms a call, B200 and its host)
+    std::vector<float> g = packGrids(*env, false);
     EnvParams E = toEnvParams(*env);
     std::lock_guard<std::mutex> lock(g_envMu);
     unsigned char* base = nullptr;
     CK(envScratch(dev, &base));
     float* dg = (float*)base;
-    EnvIo<dr_sim_state>* dio = (EnvIo<dr_sim_state>*)(base + ENV_SCRATCH_PARAMS);
+    // grids and record in one copy
+    constexpr size_t oIo = (GRID_FLOATS * 4 + 255) & ~(size_t)255;
+    static_assert(oIo + sizeof(EnvIo<dr_sim_state>) <= ENV_SCRATCH_PARAMS, "env step scratch");
+    EnvIo<dr_sim_state>* dio = (EnvIo<dr_sim_state>*)(base + oIo);
     EnvIo<dr_sim_state> io{};
     io.state = *state;
     for (int i = 0; i < env->n_theta; i++)
         io.belief[i] = belief[i];
-    CK(cudaMemcpy(dg, g.data(), GRID_FLOATS * 4, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(dio, &io, sizeof(io), cudaMemcpyHostToDevice));
+    std::vector<unsigned char> up(oIo + sizeof(io));
+    std::memcpy(up.data(), g.data(), GRID_FLOATS * 4);
+    std::memcpy(up.data() + oIo, &io, sizeof(io));
+    CK(cudaMemcpy(dg, up.data(), up.size(), cudaMemcpyHostToDevice));
     uint32_t k0 = (uint32_t)seed, k1 = (uint32_t)(seed >> 32);
     switch (env->n_opp * 16 + env->n_theta)
     {
@@ -1240,7 +1247,7 @@ extern "C" int dr_gate_env_step(const dr_gate_env_config* env, int true_theta, c
     int dev = 0;
     CK(cudaGetDevice(&dev));
     GateParams hp = toGateParams(*env);
-    std::vector<float> tr = packGateTrack(*env);
+    std::vector<float> tr = packGateTrack(*env, false);
     const size_t trOff = (sizeof(GateParams) + 255) & ~(size_t)255;
     if (trOff + tr.size() * 4 > ENV_SCRATCH_PARAMS)
         return fail(DR_ERR_INVALID_ARG, "gate parameters too large");

@@ -68,6 +68,33 @@ struct DevScratch
     }
 };
 
+// The same in pinned host memory.
+struct PinnedScratch
+{
+    void* p = nullptr;
+    size_t bytes = 0;
+    cudaError_t reserve(size_t n)
+    {
+        if (n <= bytes)
+            return cudaSuccess;
+        if (p)
+            cudaFreeHost(p);
+        p = nullptr;
+        bytes = 0;
+        cudaError_t e = cudaMallocHost(&p, n);
+        if (e == cudaSuccess)
+            bytes = n;
+        return e;
+    }
+    void release()
+    {
+        if (p)
+            cudaFreeHost(p);
+        p = nullptr;
+        bytes = 0;
+    }
+};
+
 // Bump allocator over one cudaMalloc; every block is 256-byte aligned.
 struct Arena
 {
@@ -205,7 +232,10 @@ inline float projectionCertificate(const float* P, int c)
     return r > 0.0 ? (float)(r * r * (1.0 - 1e-5)) : -1.0f;
 }
 
-inline std::vector<float> packGrids(const dr_env_config& c)
+// The track's grids in the layout of model.cuh. certificate = false leaves the projection
+// certificates out (no sample is certified, so the window is always scanned, for the same
+// result): they take the host 0.4 ms, which a controller pays once and a single step should not.
+inline std::vector<float> packGrids(const dr_env_config& c, bool certificate = true)
 {
     std::vector<float> g(GRID_FLOATS, 0.0f);
     for (int i = -GRID_PAD; i < NTS + GRID_PAD; i++)
@@ -224,7 +254,7 @@ inline std::vector<float> packGrids(const dr_env_config& c)
         g[GRID_K + i] = c.kappa_grid[k];
     }
     for (int i = 0; i < NTS; i++)
-        g[GRID_CERT + i] = projectionCertificate(c.p_grid, i);
+        g[GRID_CERT + i] = certificate ? projectionCertificate(c.p_grid, i) : -1.0f;
     return g;
 }
 
@@ -325,8 +355,9 @@ inline GateParams toGateParams(const dr_gate_env_config& c)
 }
 
 // racelines plus the sample the reference reads when s wraps to exactly 1.0f, then each
-// raceline's padded x and y rows (the gate track buffer's layout, gate_model.cuh)
-inline std::vector<float> packGateTrack(const dr_gate_env_config& c)
+// raceline's padded x and y rows (the gate track buffer's layout, gate_model.cuh);
+// certificate = false: as packGrids, no sample certified and the margins always scanned
+inline std::vector<float> packGateTrack(const dr_gate_env_config& c, bool certificate = true)
 {
     std::vector<float> t(GATE_TRACK_FLOATS, 0.0f);
     const size_t n = (size_t)G_NR * NTS * 2;
@@ -344,7 +375,7 @@ inline std::vector<float> packGateTrack(const dr_gate_env_config& c)
         }
     for (int r = 0; r < G_NR; r++)
         for (int i = 0; i < NTS; i++)
-            t[(size_t)GATE_CERT + (size_t)r * NTS + i] = projectionCertificate(c.track_points + (size_t)r * NTS * 2, i);
+            t[(size_t)GATE_CERT + (size_t)r * NTS + i] = certificate ? projectionCertificate(c.track_points + (size_t)r * NTS * 2, i) : -1.0f;
     return t;
 }
 
