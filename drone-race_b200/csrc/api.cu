@@ -50,11 +50,12 @@ struct dr_mppi
     bool exactVerify = false;
     bool egoTableOn = true; // dr_mppi_set_ego_table
 
-    // The fast verification takes the ego's moves from the ego tables: they exist, are
-    // switched on and no noise of the environment moves the ego.
+    // The fast verification takes the ego's moves from the ego tables (gate race: the
+    // clearance blocks): they exist, are switched on and no noise of the environment moves
+    // the ego.
     bool egoTableUsable() const
     {
-        return !exactVerify && egoTableOn && desc.egoTab && env.action_noise_level == 0.0f && env.pos_noise_level == 0.0f &&
+        return !exactVerify && egoTableOn && desc.clear && env.action_noise_level == 0.0f && env.pos_noise_level == 0.0f &&
                env.speed_noise_level == 0.0f;
     }
     DevScratch predBuf; // dr_mppi_predict's inputs and outputs on the device
@@ -266,7 +267,7 @@ struct dr_mppi_batch
     // every controller's verification reads its ego tables (filled before each verification)
     bool egoTable() const
     {
-        if (envKind != 0 || !verify)
+        if (!verify)
             return false;
         for (auto* h : hs)
             if (!h->egoTableUsable())
@@ -289,7 +290,8 @@ struct dr_mppi_batch
         int maxH = 1;
         for (auto* h : hs)
             maxH = std::max(maxH, h->H);
-        return launchEgoTable(s, nopp, nth, dDesc, in, (int)hs.size(), plans, maxH);
+        return envKind ? launchGateClear(s, nth, iMppi, dDesc, in, (int)hs.size(), plans, maxH)
+                       : launchEgoTable(s, nopp, nth, dDesc, in, (int)hs.size(), plans, maxH);
     }
 
     cudaError_t launchRollout(const LaunchArgs& a) const
@@ -1006,6 +1008,13 @@ static int createMppi(const dr_env_config* env, const dr_gate_env_config* genv, 
         h->env = *env;
         h->env.p_grid = h->env.dp_grid = h->env.t_grid = h->env.kappa_grid = nullptr;
     }
+    else
+    {
+        // the noise levels decide whether the verification's samples share the ego's moves
+        h->env.action_noise_level = genv->action_noise_level;
+        h->env.pos_noise_level = genv->pos_noise_level;
+        h->env.speed_noise_level = genv->speed_noise_level;
+    }
     h->cfg = *cfg;
     h->seed = seed;
     h->nth = env ? env->n_theta : genv->n_theta;
@@ -1090,9 +1099,10 @@ static int createMppi(const dr_env_config* env, const dr_gate_env_config* genv, 
     EgoRow* egoTab = nullptr;
     float* clear = nullptr;
     const size_t egoBytes = (size_t)2 * egoRows(nth, h->H) * h->H * sizeof(EgoRow);
-    if (env && cfg->verify && egoBytes <= EGO_TABLE_MAX_BYTES)
+    if (cfg->verify && egoBytes <= EGO_TABLE_MAX_BYTES)
     {
-        A.add(egoTab, egoBytes);
+        if (env)
+            A.add(egoTab, egoBytes);
         A.add(clear, (size_t)2 * clearWords(h->H) * 4);
     }
 
@@ -1803,11 +1813,12 @@ static int debugVerify(dr_mppi* h, const St* state, const float* belief, const f
         a.tiles = dT;
         a.nTiles = (int)tiles.size();
         a.exactVerify = h->exactVerify ? 1 : 0;
-        a.egoTable = h->envKind == 0 && h->egoTableUsable() ? 1 : 0;
+        a.egoTable = h->egoTableUsable() ? 1 : 0;
         if (a.egoTable) // the prologue zeroes the clearance blocks in a step
             cudaMemsetAsync(D.clear, 0, (size_t)2 * clearWords(h->H) * 4, h->stream);
         if (a.egoTable)
-            e = launchEgoTable(h->stream, h->nopp, h->nth, dD, dIn, 1, plan, h->H);
+            e = h->envKind ? launchGateClear(h->stream, h->nth, h->iMppi, dD, dIn, 1, plan, h->H)
+                           : launchEgoTable(h->stream, h->nopp, h->nth, dD, dIn, 1, plan, h->H);
         if (e == cudaSuccess)
             e = h->envKind ? launchGateVerify(a, h->nth, h->iMppi, gateVerifySmem(h->nth, T), dFt, dTh)
                        : launchMppiVerify(a, h->nopp, h->nth, mppiVerifySmem(h->nth, T), dFt, dTh);

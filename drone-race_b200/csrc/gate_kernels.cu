@@ -7,8 +7,10 @@
 // mppi_kernels.cu serve both environments (they see only costs, bookkeeping and plans).
 #include <cstdio>
 
+#include <cfloat>
 #include <type_traits>
 
+#include "clear.cuh"
 #include "common.cuh"
 #include "gate_model.cuh"
 #include "instance.cuh"
@@ -238,6 +240,123 @@ __global__ void __launch_bounds__(GRB) gate_rollout(const MppiDev* __restrict__ 
     }
 }
 
+// The clearance block of a plan (ClearBlock; plan 0 the new one, 1 the previous one, 2 both)
+// from the ego's trajectories (no branch, or a branch taken at a step: the rows of the
+// strategic race's ego tables), which need the plan alone: the controls clamped, position,
+// velocity and speed cap as gateStep takes them, up to rounding (clearOfEgo's slack). The time
+// is one trajectory's chain of steps, so GCLEAR_STEPS lanes take as many steps of a row at a
+// time: each runs the short chain, with the trajectory with no branch beside it, and then
+// judges its own step (25 -> 12 us a plan of four agents, H 40, two hypotheses, against a
+// lane per row; B200, 1965 MHz). Only for an ego that draws no noise.
+constexpr int GCLEAR = 128, GCLEAR_STEPS = 8, GCLEAR_ROWS = GCLEAR / GCLEAR_STEPS;
+
+template <int NTH, int ME>
+__global__ void __launch_bounds__(GCLEAR) gate_clear(const MppiDev* __restrict__ insts, const MppiIn* __restrict__ in, int nInst, int plans)
+{
+    __shared__ GateParams sG; // without its belief terms
+    __shared__ float2 ctl[(NTH + 1) * DR_MAX_T];
+    const int inst = blockIdx.x;
+    if (inst >= nInst)
+        return;
+    const MppiDev& D = insts[inst];
+    const MppiIn& I = in[inst];
+    if (!D.clear)
+        return;
+    const int H = D.cfg.H, T = D.cfg.T, rows = egoRows(NTH, H);
+    for (int i = threadIdx.x; i < GATE_HOST_WORDS; i += GCLEAR)
+        ((float*)&sG)[i] = ((const float*)D.gate)[i];
+    const GateParams& G = sG;
+    float belief[NTH];
+#pragma unroll
+    for (int i = 0; i < NTH; i++)
+        belief[i] = I.belief[i];
+    const int pt0 = findConfident<NTH>(belief, D.cfg.minConf);
+    const int nRows = pt0 != 0 ? 1 : rows; // a confident initial belief never branches
+    const int sub = threadIdx.x % GCLEAR_STEPS; // this lane's step
+    for (int plan = plans == 1 ? 1 : 0; plan <= (plans == 0 ? 0 : 1); plan++)
+    {
+        __syncthreads(); // the parameters, and the previous plan's rows are done with ctl
+        const float2* P = (const float2*)(plan == 0 ? D.dense : D.prevDense);
+        const float maxAccel = G.maxAccel[ME], maxSpeed = G.maxSpeed[ME], dt = G.dt;
+        for (int i = threadIdx.x; i < (NTH + 1) * T; i += GCLEAR)
+        {
+            const float2 u = P[i];
+            const float sq = u.x * u.x + u.y * u.y;
+            const float f = sq > maxAccel * maxAccel ? mdivsqrt<true>(maxAccel, sq) : 1.0f;
+            ctl[i] = make_float2(u.x * f, u.y * f);
+        }
+        __syncthreads();
+        const ClearBlock<float> cb(D.clear + (size_t)plan * clearWords(H), H);
+        auto advance = [&](float2 u, float (&p)[2], float (&v)[2]) {
+            p[0] += dt * v[0];
+            p[1] += dt * v[1];
+            v[0] += dt * u.x;
+            v[1] += dt * u.y;
+            const float sq = v[0] * v[0] + v[1] * v[1];
+            if (sq > maxSpeed * maxSpeed)
+            {
+                const float sc = mdivsqrt<true>(maxSpeed, sq);
+                v[0] *= sc;
+                v[1] *= sc;
+            }
+        };
+        for (int r = blockIdx.y * GCLEAR_ROWS + threadIdx.x / GCLEAR_STEPS; r < nRows; r += gridDim.y * GCLEAR_ROWS)
+        {
+            const int bb = r > 0 ? 1 + (r - 1) / H : 0, tb = r > 0 ? (r - 1) % H : H;
+            float p[2] = {I.gstate.pos[2 * ME], I.gstate.pos[2 * ME + 1]}, v[2] = {I.gstate.vel[2 * ME], I.gstate.vel[2 * ME + 1]};
+            float bp[2] = {p[0], p[1]}, bv[2] = {v[0], v[1]};
+            for (int t0 = 0; t0 < H; t0 += GCLEAR_STEPS)
+            {
+                const int t = t0 + sub;
+                float x = 0.0f, y = 0.0f, bx = 0.0f, by = 0.0f; // after step t
+#pragma unroll
+                for (int u = 0; u < GCLEAR_STEPS; u++)
+                {
+                    const int w = t0 + u;
+                    if (w < H)
+                    {
+                        advance(ctl[(w <= tb ? pt0 : bb) * T + (w <= tb ? w : w - tb - 1)], p, v);
+                        advance(ctl[pt0 * T + w], bp, bv);
+                    }
+                    if (u == sub)
+                    {
+                        x = p[0];
+                        y = p[1];
+                        bx = bp[0];
+                        by = bp[1];
+                    }
+                }
+                if (t >= H)
+                    continue;
+                // the ego's own boundary distance (the opponent far away), and some slack: the
+                // verification moves the ego itself
+                GState s;
+                s.pos[2 * ME] = x;
+                s.pos[2 * ME + 1] = y;
+                s.pos[2 * (1 - ME)] = s.pos[2 * (1 - ME) + 1] = INFINITY;
+                const bool off = !(gateBoundaryDist<ME, true>(s, G) >= G.droneRadius + 2e-3f + 4.8e-7f * (float)H * (fabsf(x) + fabsf(y)));
+                if (r == 0)
+                {
+                    cb.xy[2 * t] = x;
+                    cb.xy[2 * t + 1] = y;
+                    if (off)
+                        *cb.out = 1.0f;
+                }
+                else if (t > tb) // up to its branching step a row is the first one
+                {
+                    // off the arena, or a distance that is no number: infinitely far
+                    float d = msqrt<true>((x - bx) * (x - bx) + (y - by) * (y - by));
+                    if (off || !(d <= FLT_MAX))
+                        d = INFINITY;
+                    // distances are not negative: they order as their words
+                    atomicMax((unsigned*)&cb.all[t], __float_as_uint(d));
+                    atomicMax((unsigned*)&cb.rho[tb / clearPer(H) * H + t], __float_as_uint(d));
+                }
+            }
+        }
+    }
+}
+
 // verifyNominalFailureKernel (kernels.cu:488-551) on the gate race:
 // environmentStep<true, true, false, false>; one thread per sample, both plans in one
 // grid, the CTA's warps in step (a barrier per step) as in mppi_verify.
@@ -254,7 +373,12 @@ template <int NTH> constexpr int gateVerifyMinBlocks()
 // FAST: the verification's fast arithmetic flavour and noise source (the default; the
 // exact flavour reproduces the oracle's per-sample results and serves parity tests), as
 // in the strategic race's mppi_verify; its warps step without a CTA barrier.
-template <int NTH, int ME, bool FAST>
+// CLEAR (with FAST): warps whose samples can no longer collide leave, and tiles none of whose
+// samples can end at once, by the plan's clearance block (gate_clear, clearOfEgo), as in
+// mppi_verify; a sample fails at the first step with boundary distance below the drone radius,
+// which the ego's own part of that distance, known with its trajectory, and the opponents'
+// distance decide.
+template <int NTH, int ME, bool FAST, bool CLEAR = false>
 __global__ void __launch_bounds__(VERIFY_TILE, (gateVerifyMinBlocks<NTH>())) gate_verify(const MppiDev* __restrict__ insts, const MppiIn* __restrict__ in, const Tile* __restrict__ tiles,
                                                              int* __restrict__ dbgFailTime, int* __restrict__ dbgTheta)
 {
@@ -271,15 +395,29 @@ __global__ void __launch_bounds__(VERIFY_TILE, (gateVerifyMinBlocks<NTH>())) gat
     float* sTrack = (float*)(smraw + offT);
     float* sPlan = (float*)(smraw + offT + GATE_TRACK_FLOATS * 4);
     const uint32_t planBytes = (uint32_t)ga16((size_t)NBP * T * 2 * 4);
-    unsigned* hist = (unsigned*)(smraw + offT + GATE_TRACK_FLOATS * 4 + planBytes);
+    const uint32_t clearBytes = CLEAR ? (uint32_t)clearWords(H) * 4u : 0u;
+    float* sClear = (float*)(smraw + offT + GATE_TRACK_FLOATS * 4 + planBytes);
+    unsigned* hist = (unsigned*)((unsigned char*)sClear + clearBytes);
+    constexpr int opp = 1 - ME;
+    if constexpr (CLEAR)
+    {
+        // every sample starts from the same state
+        const ClearBlock<const float> cb(D.clear + (size_t)plan * clearWords(H), H);
+        if (!dbgTheta && *cb.out == 0.0f &&
+            clearOfEgo(D.gate->dt, D.gate->droneRadius, cb.xy, cb.all, H, 0, true, I.gstate.pos[2 * opp], I.gstate.pos[2 * opp + 1], I.gstate.vel[2 * opp],
+                       I.gstate.vel[2 * opp + 1], D.gate->maxSpeed[opp], D.gate->maxAccel[opp]))
+            return;
+    }
     if (threadIdx.x == 0)
     {
         mbar_init(bar, 1);
-        mbar_expect_tx(bar, GATE_TRACK_FLOATS * 4 + planBytes);
+        mbar_expect_tx(bar, GATE_TRACK_FLOATS * 4 + planBytes + clearBytes);
         if (!D.cfg.dbgNoStage)
         {
             bulk_g2s(sTrack, D.gtrack, GATE_TRACK_FLOATS * 4, bar);
             bulk_g2s(sPlan, plan == 0 ? D.dense : D.prevDense, planBytes, bar);
+            if (CLEAR)
+                bulk_g2s(sClear, D.clear + (size_t)plan * clearWords(H), clearBytes, bar);
         }
     }
     copyGate(sG, D.gate);
@@ -291,6 +429,11 @@ __global__ void __launch_bounds__(VERIFY_TILE, (gateVerifyMinBlocks<NTH>())) gat
         if (threadIdx.x == 0)
             atomicAdd(&D.stats[1], 1);
         return;
+    }
+    if constexpr (CLEAR)
+    {
+        clearSuffix(sClear, H);
+        __syncthreads();
     }
     const GateParams& G = *sG;
     const int v = tile.s0 + threadIdx.x;
@@ -306,6 +449,7 @@ __global__ void __launch_bounds__(VERIFY_TILE, (gateVerifyMinBlocks<NTH>())) gat
             bs.belief[i] = I.belief[i];
         bs.predTheta = findConfident<NTH>(bs.belief, minConf);
         bs.branchingTime = bs.predTheta == 0 ? -1 : 0;
+        const int pt0 = bs.predTheta;
         // sampleModelFromBelief (state.h:118-131) on a Philox uniform
         const uint32_t k0 = D.cfg.k0, k1 = D.cfg.k1, step = I.step;
         float u = uniform_from_word(draw(k0, k1, (uint32_t)v, (uint32_t)plan, step, S_VERIF_THETA, 0).x);
@@ -341,6 +485,17 @@ __global__ void __launch_bounds__(VERIFY_TILE, (gateVerifyMinBlocks<NTH>())) gat
             }
             else if (!__syncthreads_or(active))
                 break;
+            if constexpr (CLEAR)
+                if (t % CLEAR_EVERY == 0)
+                {
+                    // the group of the earliest branch that a sample has taken or can take
+                    const int tau = bs.predTheta == 0 || pt0 != 0 ? t : tOrigin - 1;
+                    const int gr = __reduce_min_sync(0xffffffffu, active ? (unsigned)tau : ~0u) / (unsigned)clearPer(H);
+                    const ClearBlock<const float> cb(sClear, H);
+                    if (*cb.out == 0.0f && clearOfEgo(G.dt, G.droneRadius, cb.xy, cb.rho + gr * H, H, t, active, st.pos[2 * opp], st.pos[2 * opp + 1],
+                                                      st.vel[2 * opp], st.vel[2 * opp + 1], G.maxSpeed[opp], G.maxAccel[opp]))
+                        break;
+                }
             if (!active)
                 continue;
             rng.begin_step((uint32_t)t);
@@ -471,7 +626,9 @@ size_t gateRolloutSmem(int nth, int T, int M, bool spl)
 
 size_t gateVerifySmem(int nth, int T)
 {
-    return ga16(16 + sizeof(GateParams)) + GATE_TRACK_FLOATS * 4 + ga16((size_t)(nth + 1) * T * 2 * 4) + (size_t)T * 4;
+    // the clearance block of the longest verification horizon, T
+    return ga16(16 + sizeof(GateParams)) + GATE_TRACK_FLOATS * 4 + ga16((size_t)(nth + 1) * T * 2 * 4) + ((size_t)T * (3 + CLEAR_GROUPS) + 4) * 4 +
+           (size_t)T * 4;
 }
 
 int gateRolloutSamplesPerBlock(int nth)
@@ -498,7 +655,7 @@ template <int NTH, int ME> static cudaError_t launchGateRolloutT(const LaunchArg
 
 template <int NTH, int ME> static cudaError_t launchGateVerifyT(const LaunchArgs& a, size_t smem, int* ft, int* th)
 {
-    auto k = a.exactVerify ? gate_verify<NTH, ME, false> : gate_verify<NTH, ME, true>;
+    auto k = a.exactVerify ? gate_verify<NTH, ME, false> : a.egoTable ? gate_verify<NTH, ME, true, true> : gate_verify<NTH, ME, true>;
     ensureSmem(k, smem);
     k<<<a.nTiles, VERIFY_TILE, smem, a.stream>>>(a.mppi, a.mppiIn, a.tiles, ft, th);
     return cudaGetLastError();
@@ -522,6 +679,21 @@ template <int NTH, int ME> static cudaError_t launchGateVerifyT(const LaunchArgs
 cudaError_t launchGateRollout(const LaunchArgs& a, int nth, int me, bool spl, size_t smem)
 {
 #define CALL(P, Q) launchGateRolloutT<P, Q>(a, spl, smem)
+    GATE_DISPATCH(nth, me, CALL)
+#undef CALL
+}
+
+template <int NTH, int ME>
+static cudaError_t launchGateClearT(cudaStream_t stream, const MppiDev* insts, const MppiIn* in, int nInst, int plans, int maxH)
+{
+    const dim3 grid(nInst, (unsigned)((egoRows(NTH, maxH) + GCLEAR_ROWS - 1) / GCLEAR_ROWS));
+    gate_clear<NTH, ME><<<grid, GCLEAR, 0, stream>>>(insts, in, nInst, plans);
+    return cudaGetLastError();
+}
+
+cudaError_t launchGateClear(cudaStream_t stream, int nth, int me, const MppiDev* insts, const MppiIn* in, int nInst, int plans, int maxH)
+{
+#define CALL(P, Q) launchGateClearT<P, Q>(stream, insts, in, nInst, plans, maxH)
     GATE_DISPATCH(nth, me, CALL)
 #undef CALL
 }

@@ -33,7 +33,8 @@ struct LaunchArgs
     // with the oracle), 0 = the fast flavour (the default)
     int exactVerify = 0;
     // fast verification: 1 = the ego's moves come from the instances' ego tables
-    // (mppi_ego_table must have filled them for the plans verified)
+    // (mppi_ego_table must have filled them for the plans verified); gate race: 1 = the
+    // clearance blocks are filled (gate_clear)
     int egoTable = 0;
     // PR-MPPI rollout: hypothesis slots per thread (1, 2, 4), sharing the ego's moves
     int prSlots = 1;
@@ -89,6 +90,8 @@ int gateRolloutSamplesPerBlock(int nth);
 size_t gateRolloutSmem(int nth, int T, int M, bool spl);
 size_t gateVerifySmem(int nth, int T);
 // `me`: the ego's agent index (the environment's i_mppi)
+// fills the clearance blocks (MppiDev::clear) of plan `plans` (0 new, 1 previous, 2 both)
+cudaError_t launchGateClear(cudaStream_t stream, int nth, int me, const MppiDev* insts, const MppiIn* in, int nInst, int plans, int maxH);
 cudaError_t launchGateRollout(const LaunchArgs& a, int nth, int me, bool spl, size_t smem);
 cudaError_t launchGateVerify(const LaunchArgs& a, int nth, int me, size_t smem, int* dbgFailTime, int* dbgTheta);
 cudaError_t launchGateBatchEnvStep(cudaStream_t stream, int nth, int me, const MppiDev* insts, const MppiIn* in, int nInst, const int* trueTheta,

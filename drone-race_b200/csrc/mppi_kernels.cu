@@ -26,6 +26,7 @@
 #include <cstdio>
 #include <type_traits>
 
+#include "clear.cuh"
 #include "common.cuh"
 #include "instance.cuh"
 #include "launch.h"
@@ -1126,65 +1127,6 @@ __global__ void __launch_bounds__(UB) mppi_shard_apply(const MppiDev* __restrict
 // it does not, the steps are taken one by one (egoStep). The lane also runs the trajectory
 // with no branch beside its own and puts its distance from it into the clearance block.
 constexpr int EGO_WARPS = 4;
-// Steps between two clearance tests of a verification warp: a test costs about 60
-// instructions, a step about 700. Four agents of 2 x 2^17 x 40, three drawn mid-race states
-// (B200, 1965 MHz; the verification of the new plan): without the test 0.52 / 0.45 / 0.55 ms,
-// every step 0.36 / 0.27 / 0.08, every second 0.35 / 0.26 / 0.08, every fourth 0.35 / 0.25 /
-// 0.10.
-#ifndef DR_CLEAR_EVERY
-#define DR_CLEAR_EVERY 2
-#endif
-constexpr int CLEAR_EVERY = DR_CLEAR_EVERY;
-
-// Whether no remaining step (t .. H - 1) of the warp's active samples can bring an opponent
-// within two drone radii of the ego, or the ego off the track: then none of them can fail any
-// more (a sample fails at the first step with boundary distance below the drone radius) and
-// their remaining steps decide nothing. px .. vy: this lane's opponent before step t; xy: the
-// ego's trajectory with no branch (which stays on the track), rho: how far the samples' own may
-// be from it, after each step.
-//
-// An opponent whose speed is within its limit vmax moves k dt v in k steps plus at most
-// amax dt^2 k (k - 1) / 2: the step moves it by its velocity before the step and then adds an
-// acceleration clamped to amax, and the cap to vmax, a projection onto a ball that holds the
-// old velocity, never moves the new one farther from it. The warp's opponents lie within
-// (dp, dv) of the first active lane's in position and velocity (1-norms, which bound the
-// Euclidean ones). The ego is on a row of its table: within rho of the trajectory with no
-// branch. So after step j the two are at least |ego_j - (p + k dt v)| - rho - dp - k dt dv -
-// amax dt^2 k (k - 1) / 2 apart, k = j - t + 1. Slack for the arithmetic (the verification's
-// approximate factors are within 1e-5, positions round to 2^-24 a step): a millimetre, 1e-4 of
-// the reach and of the speed limit's way, and H roundings of the coordinates.
-__device__ __forceinline__ bool clearOfEgo(const EnvParams& E, const float* xy, const float* rho, int H, int t, bool active, float px, float py, float vx,
-                                           float vy, float vmax, float amax)
-{
-    vmax = fabsf(vmax);
-    amax = fabsf(amax);
-    constexpr unsigned ALL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    const int src = __ffs(__ballot_sync(ALL, active)) - 1;
-    const float cx = __shfl_sync(ALL, px, src), cy = __shfl_sync(ALL, py, src), wx = __shfl_sync(ALL, vx, src), wy = __shfl_sync(ALL, vy, src);
-    float dp = 0.0f, dv = 0.0f;
-    bool ok = true;
-    if (active)
-    {
-        dp = fabsf(px - cx) + fabsf(py - cy);
-        dv = fabsf(vx - wx) + fabsf(vy - wy);
-        ok = vx * vx + vy * vy <= vmax * vmax * 1.0001f;
-    }
-    // non-negative floats (and NaN, above them all) order as their words
-    dp = __uint_as_float(__reduce_max_sync(ALL, __float_as_uint(dp)));
-    dv = __uint_as_float(__reduce_max_sync(ALL, __float_as_uint(dv)));
-    for (int j = t + lane; j < H; j += 32)
-    {
-        const float k = (float)(j - t + 1), kd = k * E.dt;
-        const float ex = xy[2 * j] - (cx + kd * wx), ey = xy[2 * j + 1] - (cy + kd * wy);
-        const float way = kd * vmax;
-        const float reach = 2.0f * E.droneRadius + rho[j] + dp + kd * dv + 0.5f * amax * E.dt * E.dt * (k * (k - 1.0f));
-        const float slack = 1e-3f + 1e-4f * (reach + way) + 2.4e-7f * (float)H * (fabsf(cx) + fabsf(cy) + way);
-        const float need = reach + slack;
-        ok = ok && ex * ex + ey * ey > need * need;
-    }
-    return __all_sync(ALL, ok);
-}
 
 // 8 / 16 / 32 steps at a time: 18.5 / 17.0 / 16.6 us for a plan of four agents, H 40, two
 // hypotheses (B200, 1965 MHz); more steps repeat more of the short chain, which large batches
@@ -1491,7 +1433,7 @@ __global__ void __launch_bounds__(VERIFY_TILE, (verifyMinBlocks<NOPP, NTH>())) m
             const ClearBlock<const float> cb(D.clear + (size_t)plan * clearWords(H), H);
             clear = clear && *cb.out == 0.0f;
             for (int o = 1; o <= NOPP; o++)
-                clear = clear && clearOfEgo(D.env, cb.xy, cb.all, H, 0, true, I.state.pos[2 * o], I.state.pos[2 * o + 1], I.state.vel[2 * o],
+                clear = clear && clearOfEgo(D.env.dt, D.env.droneRadius, cb.xy, cb.all, H, 0, true, I.state.pos[2 * o], I.state.pos[2 * o + 1], I.state.vel[2 * o],
                                             I.state.vel[2 * o + 1], D.env.maxSpeed[o], D.env.maxAccel[o]);
             if (clear)
             {
@@ -1531,11 +1473,7 @@ __global__ void __launch_bounds__(VERIFY_TILE, (verifyMinBlocks<NOPP, NTH>())) m
             staged = key;
             if constexpr (EGO)
             {
-                // from each group's own distances to those of it and the later ones
-                const ClearBlock<float> cb(sClear, H);
-                for (int j = threadIdx.x; j < H; j += blockDim.x)
-                    for (int g = clearGroups(H) - 2; g >= 0; g--)
-                        cb.rho[g * H + j] = fmaxf(cb.rho[g * H + j], cb.rho[(g + 1) * H + j]);
+                clearSuffix(sClear, H);
                 __syncthreads();
             }
         }
@@ -1605,7 +1543,7 @@ __global__ void __launch_bounds__(VERIFY_TILE, (verifyMinBlocks<NOPP, NTH>())) m
                         bool clear = *cb.out == 0.0f;
 #pragma unroll
                         for (int o = 1; o <= NOPP; o++)
-                            clear = clear && clearOfEgo(E, cb.xy, cb.rho + gr * H, H, t, active, st.pos[2 * o], st.pos[2 * o + 1], st.vel[2 * o],
+                            clear = clear && clearOfEgo(E.dt, E.droneRadius, cb.xy, cb.rho + gr * H, H, t, active, st.pos[2 * o], st.pos[2 * o + 1], st.vel[2 * o],
                                                         st.vel[2 * o + 1], E.maxSpeed[o], E.maxAccel[o]);
                         if (clear)
                             break;

@@ -76,3 +76,32 @@ def test_clear_tiles_of_whole_steps(gpu):
             out.append(r)
         for a, b in zip(*out):
             assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("me", [0, 1])
+@pytest.mark.parametrize("Hv", [7, 8, 9, 40, 41, 60])
+@pytest.mark.parametrize("gap,toward", [(0.016, True), (0.02, True), (0.02, False), (0.035, True), (0.05, False), (0.2, False)])
+def test_gate_clearance_changes_no_failure(gpu, me, Hv, gap, toward):
+    """The same on the gate race (gate_clear): an obstacle beside the track, either agent as the
+    ego, horizons around the steps that a lane group takes."""
+    import helpers as H
+
+    sc = H.small_gate(False, K=64, T=60, n_verif=1100, seed=3)
+    sc.mppi.verif_horizon = Hv
+    sc.env.i_mppi = me
+    u = [0.31, 0.31 + gap] if me == 0 else [0.31 + gap, 0.31]
+    sc.state = S.gate_state(sc.track, u, me, [0, 0], speed=3.0)
+    sc.env.n_round_obstacles = 1
+    sc.env.round_obs_centers[0], sc.env.round_obs_centers[1], sc.env.round_obs_radius[0] = 2.0, 7.0, 0.4
+    rng = np.random.default_rng(Hv)
+    plan = H.toward_opponent_plan(sc) if toward else rng.normal(0, 3.0, (3, 60, 2)).astype(np.float32)
+    out = []
+    for table in (True, False):
+        ctl = drb.controllers.MPPIController(sc.env, sc.mppi, 5)
+        ctl.set_ego_table(table)
+        fc, ft = np.zeros(60, np.uint32), np.zeros(1100, np.int32)
+        abi.check(abi.lib().dr_gate_mppi_debug_verify(ctl.handle, C.byref(sc.state), abi.fptr(sc.belief()), abi.fptr(plan), 1, abi.uptr(fc),
+                                                      abi.iptr(ft), None), "gate debug_verify")
+        out.append((fc, ft))
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
