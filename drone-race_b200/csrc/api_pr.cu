@@ -17,6 +17,7 @@
 #include "hostutil.hpp"
 #include "instance.cuh"
 #include "launch.h"
+#include "pr_split.cuh"
 
 using namespace dr;
 
@@ -137,6 +138,7 @@ struct dr_prmppi_batch
     PrIn* hIn = nullptr;
     Tile *dRoll = nullptr, *dWa = nullptr;
     int nRoll = 0, nWa = 0;
+    int prThreads = PRS_TILE; // threads of a rollout CTA that shares egos (prTileThreads)
     size_t rollSmem = 0;
     bool useGraph = true;
     bool profiling = false;
@@ -156,7 +158,7 @@ struct dr_prmppi_batch
     // draws no noise (its moves are then shared by the slots) and P is a multiple
     int slotsFor(int want) const
     {
-        if (!egoShared() || want <= 1)
+        if (envKind != 0 || !egoShared() || want <= 1)
             return 1;
         for (auto* h : hs)
             if (h->P % want != 0)
@@ -164,11 +166,9 @@ struct dr_prmppi_batch
         return want;
     }
 
-    // no controller's ego draws noise (strategic race)
+    // no controller's ego draws noise
     bool egoShared() const
     {
-        if (envKind != 0)
-            return false;
         for (auto* h : hs)
             if (h->env.action_noise_level != 0.0f || h->env.pos_noise_level != 0.0f || h->env.speed_noise_level != 0.0f)
                 return false;
@@ -193,6 +193,7 @@ struct dr_prmppi_batch
         a.nTiles = n;
         a.prSlots = slotsFor(prSlots);
         a.prShared = egoShared() ? 1 : 0;
+        a.prThreads = prThreads;
         return a;
     }
 
@@ -213,7 +214,7 @@ struct dr_prmppi_batch
         CK(launchPrReduce(args(dWa, nWa, in), maxSamples()));
         if (profile)
             timer->mark("candidates", stream);
-        CK(envKind ? launchGatePrCandidates(args(nullptr, 0, in), nth, iMppi, n, maxT) : launchPrCandidates(args(nullptr, 0, in), nopp, nth, n, maxT, maxP));
+        CK(envKind ? launchGatePrCandidates(args(nullptr, 0, in), nth, iMppi, n, maxT, maxP) : launchPrCandidates(args(nullptr, 0, in), nopp, nth, n, maxT, maxP));
         if (profile)
         {
             timer->mark("end", stream);
@@ -412,6 +413,26 @@ struct dr_prmppi_batch
 namespace
 {
 
+// Threads of a rollout CTA that shares egos: 512, two CTAs of which fill an SM, or fewer while
+// the launch would leave SMs without one (one gate-race agent of 2 x 8 x 2048 samples: 74 CTAs
+// of 512 threads or 148 of 256, 0.171 / 0.154 ms; B200, 1965 MHz).
+int prTileThreads(dr_prmppi* const* hs, int n)
+{
+    int threads = PRS_TILE;
+    for (; threads > PRS_MIN_TILE; threads /= 2)
+    {
+        long long tiles = 0;
+        for (int i = 0; i < n; i++)
+        {
+            const int spb = hs[i]->envKind ? gatePrRolloutSamplesPerTile(hs[i]->P, threads) : prRolloutSamplesPerTile(hs[i]->P, threads);
+            tiles += 2LL * ((hs[i]->sHi - hs[i]->sLo + spb - 1) / spb);
+        }
+        if (tiles >= 148)
+            break;
+    }
+    return threads;
+}
+
 int buildPrBatch(dr_prmppi* const* hs, int n, cudaStream_t stream, bool ownStream, dr_prmppi_batch** out)
 {
     if (n <= 0 || !hs)
@@ -432,11 +453,13 @@ int buildPrBatch(dr_prmppi* const* hs, int n, cudaStream_t stream, bool ownStrea
     b->ownStream = ownStream;
     std::vector<PrDev> descs;
     std::vector<Tile> roll, wa;
+    if (b->nopp == 1 && b->egoShared())
+        b->prThreads = prTileThreads(hs, n);
     for (int i = 0; i < n; i++)
     {
         dr_prmppi* h = hs[i];
         descs.push_back(h->desc);
-        const int spb = h->envKind ? gatePrRolloutSamplesPerBlock() / h->P : prRolloutSamplesPerTile(h->P);
+        const int spb = h->envKind ? gatePrRolloutSamplesPerTile(h->P, b->prThreads) : prRolloutSamplesPerTile(h->P, b->prThreads);
         for (int nr = 0; nr < 2; nr++)
             for (int s0 = h->sLo; s0 < h->sHi; s0 += spb)
                 roll.push_back(Tile{i, s0, std::min(spb, h->sHi - s0), nr});
@@ -444,7 +467,7 @@ int buildPrBatch(dr_prmppi* const* hs, int n, cudaStream_t stream, bool ownStrea
             wa.push_back(Tile{i, w, 0, 0});
         b->maxT = std::max(b->maxT, h->T);
         b->maxP = std::max(b->maxP, h->P);
-        b->rollSmem = std::max(b->rollSmem, h->envKind ? gatePrRolloutSmem(h->T) : prRolloutSmem(h->T, h->P));
+        b->rollSmem = std::max(b->rollSmem, h->envKind ? gatePrRolloutSmem(h->T, h->P) : prRolloutSmem(h->T, h->P));
     }
     b->nRoll = (int)roll.size();
     b->nWa = (int)wa.size();
@@ -501,6 +524,10 @@ static int prCreate(const dr_env_config* env, const dr_gate_env_config* genv, co
     {
         h->envKind = 1;
         h->iMppi = genv->i_mppi;
+        // the noise levels decide whether the hypotheses share the ego's moves
+        h->env.action_noise_level = genv->action_noise_level;
+        h->env.pos_noise_level = genv->pos_noise_level;
+        h->env.speed_noise_level = genv->speed_noise_level;
     }
     h->cfg = *cfg;
     if (h->cfg.min_nu == 0.0f && h->cfg.max_nu == 0.0f)

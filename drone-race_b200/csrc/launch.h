@@ -41,6 +41,7 @@ struct LaunchArgs
     // PR-MPPI: 1 = no controller's ego draws noise, so that its moves are the same under every
     // hypothesis and the kernels step it once for them
     int prShared = 0;
+    int prThreads = 512; // threads of a rollout CTA that shares egos
 };
 
 inline int launchGrid(const LaunchArgs& a)
@@ -123,10 +124,10 @@ int gradDefaultStride(int nopp, int nth, int T, int M, bool spl);
 cudaError_t launchGradNominal(cudaStream_t stream, const GradJob* jobs, int nJobs, int nopp, int nth, bool spl, size_t smem);
 
 // PR-MPPI on the gate race (gate_pr_kernels.cu); prologue and weighted averages are shared
-size_t gatePrRolloutSmem(int T);
-int gatePrRolloutSamplesPerBlock();
+size_t gatePrRolloutSmem(int T, int P);
+int gatePrRolloutSamplesPerTile(int P, int threads);
 cudaError_t launchGatePrRollout(const LaunchArgs& a, int nth, int me, size_t smem);
-cudaError_t launchGatePrCandidates(const LaunchArgs& a, int nth, int me, int nInst, int maxT);
+cudaError_t launchGatePrCandidates(const LaunchArgs& a, int nth, int me, int nInst, int maxT, int maxP);
 
 // sample-sharded PR-MPPI update phases (one controller's samples split across processes)
 cudaError_t launchPrShardMin(cudaStream_t stream, const PrDev* insts, float* mins);
@@ -168,7 +169,7 @@ cudaError_t launchCp(cudaStream_t stream, const uint32_t* k, int n, uint32_t N, 
 cudaError_t launchTrackGrids(cudaStream_t stream, const double* q, int nTracks, float* out, float* lengths);
 
 bool prSupported(int nopp, int nth);
-int prRolloutSamplesPerTile(int P);
+int prRolloutSamplesPerTile(int P, int threads);
 size_t prRolloutSmem(int T, int P);
 cudaError_t launchPrPrologue(const LaunchArgs& a, int nInst);
 cudaError_t launchPrRollout(const LaunchArgs& a, int nopp, int nth, size_t smem);

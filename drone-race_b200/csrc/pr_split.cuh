@@ -1,0 +1,35 @@
+// How a PR-MPPI rollout CTA that shares one ego per sample splits its threads: whole warps that
+// step an opponent each, one per (sample, hypothesis), then whole warps that step an ego each,
+// one per sample (pr_rollout_shared, gate_pr_rollout_shared).
+#pragma once
+
+namespace dr
+{
+
+constexpr int PRS_TILE = 512;     // threads of a CTA, unless the launch is small (prTileThreads)
+#ifndef DR_PRS_MIN_TILE
+#define DR_PRS_MIN_TILE 128
+#endif
+constexpr int PRS_MIN_TILE = DR_PRS_MIN_TILE; // fewest
+
+struct PrSplit
+{
+    int samples; // a tile's
+    int opp;     // threads that step opponents: whole warps
+};
+
+__host__ __device__ inline int prWarps(int threads)
+{
+    return (threads + 31) & ~31;
+}
+
+// the most samples, up to `most`, whose opponents and egos fit `threads` threads
+__host__ __device__ inline PrSplit prSplit(int P, int threads, int most)
+{
+    int n = threads / P < most ? threads / P : most;
+    while (n > 1 && prWarps(n * P) + prWarps(n) > threads)
+        n--;
+    return PrSplit{n, prWarps(n * P)};
+}
+
+} // namespace dr

@@ -24,6 +24,7 @@
 #include "instance.cuh"
 #include "launch.h"
 #include "pair_model.cuh"
+#include "pr_split.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -366,30 +367,13 @@ __global__ void __launch_bounds__(PR_ROLL_TILE / HPT, prRollMinBlocks<NOPP>()) p
 // ---------------------------------------------------------------------------------------
 // rollout with one ego per sample (one opponent, an ego that draws no noise)
 // ---------------------------------------------------------------------------------------
-// A CTA of PRS_TILE threads: PrSplit::opp threads step an opponent each, one per (sample,
-// hypothesis), and the warps after them an ego each, one per sample, a step ahead of the
-// opponents (two rows of shared memory, the step's barrier in between).
-constexpr int PRS_TILE = 512;
-
-struct PrSplit
+// PrSplit::opp threads step an opponent each, one per (sample, hypothesis), and the warps after
+// them an ego each, one per sample, a step ahead of the opponents (two rows of shared memory,
+// the step's barrier in between).
+// most samples of a tile: what the tiles of the general kernel hold
+__host__ __device__ inline PrSplit prSplitOf(int P, int threads)
 {
-    int samples; // a tile's
-    int opp;     // threads that step opponents: whole warps
-};
-
-__host__ __device__ inline int prWarps(int threads)
-{
-    return (threads + 31) & ~31;
-}
-
-// the most samples whose opponents and egos fit PRS_TILE threads, and at most as many as the
-// tiles of the general kernel hold
-__host__ __device__ inline PrSplit prSplit(int P)
-{
-    int n = PR_ROLL_TILE / P;
-    while (prWarps(n * P) + prWarps(n) > PRS_TILE)
-        n--;
-    return PrSplit{n, prWarps(n * P)};
+    return prSplit(P, threads, PR_ROLL_TILE / P);
 }
 
 struct PrsSmem
@@ -397,11 +381,10 @@ struct PrsSmem
     size_t env, grids, nom, rows, red, total;
 };
 
-__host__ __device__ inline PrsSmem prsLayout(int T, int P)
+__host__ __device__ inline PrsSmem prsLayout(int T, int P, int n)
 {
     auto a16 = [](size_t x) { return (x + 15) & ~(size_t)15; };
     PrsSmem L;
-    const size_t n = prSplit(P).samples;
     size_t off = 16;
     L.env = off;
     off = a16(off + sizeof(EnvParams));
@@ -410,9 +393,9 @@ __host__ __device__ inline PrsSmem prsLayout(int T, int P)
     L.nom = off;
     off = a16(off + (size_t)T * 2 * 4);
     L.rows = off;
-    off = a16(off + 2 * EGO_FIELDS * n * 4);
+    off = a16(off + (size_t)2 * EGO_FIELDS * n * 4);
     L.red = off;
-    off = a16(off + n * P * 2 * 4);
+    off = a16(off + (size_t)n * P * 2 * 4);
     L.total = off;
     return L;
 }
@@ -433,8 +416,8 @@ __global__ void __launch_bounds__(PRS_TILE, 2) pr_rollout_shared(const PrDev* __
     const PrIn& I = in[tile.inst];
     const int K = D.cfg.K, T = D.cfg.T, P = D.cfg.P;
     const int robust = tile.aux;
-    const PrSplit split = prSplit(P);
-    const PrsSmem L = prsLayout(T, P);
+    const PrSplit split = prSplitOf(P, blockDim.x);
+    const PrsSmem L = prsLayout(T, P, split.samples);
     uint64_t* bar = (uint64_t*)smraw;
     EnvParams* sE = (EnvParams*)(smraw + L.env);
     float* sGrid = (float*)(smraw + L.grids);
@@ -1194,14 +1177,14 @@ bool prSupported(int nopp, int nth)
     return key == 17 || key == 18 || key == 20 || key == 24 || key == 34;
 }
 
-int prRolloutSamplesPerTile(int P)
+int prRolloutSamplesPerTile(int P, int threads)
 {
-    return prSplit(P).samples;
+    return prSplitOf(P, threads).samples;
 }
 
 size_t prRolloutSmem(int T, int P)
 {
-    const size_t a = prLayout(T).total, b = prsLayout(T, P).total;
+    const size_t a = prLayout(T).total, b = prsLayout(T, P, prSplitOf(P, PRS_TILE).samples).total;
     return a > b ? a : b;
 }
 
@@ -1234,7 +1217,7 @@ template <int NOPP, int NTH> static cudaError_t prRollT(const LaunchArgs& a, siz
         {
             auto k = pr_rollout_shared;
             ensureSmem(k, smem);
-            k<<<a.nTiles, PRS_TILE, smem, a.stream>>>(a.pr, a.prIn, a.tiles);
+            k<<<a.nTiles, a.prThreads, smem, a.stream>>>(a.pr, a.prIn, a.tiles);
             return cudaGetLastError();
         }
     switch (a.prSlots)

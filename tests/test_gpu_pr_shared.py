@@ -54,3 +54,38 @@ def test_shared_ego_kernels_equal_the_general_ones(gpu, nth, P, K, noise):
         batch.close()
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("noise", [True, False])
+@pytest.mark.parametrize("me,P,K,tracked", [(0, 1, 70, False), (1, 3, 43, False), (0, 8, 29, True), (1, 9, 200, True), (0, 32, 7, False)])
+def test_gate_shared_ego_kernels_equal_the_general_ones(gpu, me, P, K, tracked, noise):
+    """The same on the gate race. An action noise of 1e-30 sends the ego's controller to the general
+    kernels and moves nothing (it is far below the last bit of any action)."""
+    import helpers as H
+
+    out = []
+    for level in (0.0, 1e-30):
+        sc = H.small_gate(False, K=K, T=40, seed=9, noise=noise)
+        sc.env.i_mppi = me
+        u = [0.22, 0.24] if me == 0 else [0.24, 0.22]
+        sc.state = S.gate_state(sc.track, u, me, [0, 0], speed=2.5)
+        if tracked:
+            for r in range(abi.DR_GATE_RACELINES):
+                sc.state.S[me * abi.DR_GATE_RACELINES + r] = float(np.float32(u[me]))
+        for th in range(2):
+            sc.env.opp_pid[th].repulsion_factor = 0.3 * th
+        sc.env.action_noise_level = level
+        sc.prmppi = S.make_prmppi(K=K, T=40, P=P)
+        sc.prmppi.final_opp_adv_weight = 15.0
+        rng = np.random.default_rng(6)
+        ctl = drb.controllers.PRMPPIController(sc.env, sc.prmppi, 5, nominal=rng.normal(0, 2.0, (40, 2)).astype(np.float32))
+        ctl.engine = object()
+        r = []
+        for _ in range(3):
+            r.append(ctl.getControl(sc.state))
+            r += list(ctl.nominals())
+            i = ctl.info
+            r.append(np.array([i.use_nom_plan, i.reset_nom, *i.cand_cost, *i.min_costs, *i.nu, *i.inv_temperature, i.nonfinite_costs]))
+        out.append(r)
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
