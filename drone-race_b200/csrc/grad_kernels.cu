@@ -12,8 +12,9 @@
 //
 //   grad_nominal   one thread-block cluster per (instance, start point), one CTA of the
 //                  cluster per hypothesis, GW warps per CTA.
-//     forward  warp 0 rolls the hypothesis out (values only) and keeps the state every
-//              `ckpt` steps (every step when ckpt == 1) in shared memory;
+//     forward  warp 0 rolls the hypothesis out (values only; its lanes share the work of a
+//              step, gstepLanes) and keeps the state every `ckpt` steps (every step when
+//              ckpt == 1) in shared memory;
 //     reverse  adjoint sweep, last segment first. A segment between two checkpoints is
 //              recomputed from its checkpoint; its steps are then taken GW at a time: warp
 //              p evaluates step t0 + p with lane j's input seeded — state component j, or
@@ -173,6 +174,36 @@ template <int NA, int NTH> __device__ __forceinline__ void storeColumn(float* co
     col[i] = costTangent;
 }
 
+// A value-only rollout by one warp: with one opponent over its lanes (gstepLanes), else alike on
+// all of them.
+template <int NOPP, int NTH> struct ValueRollout
+{
+    XState<NOPP + 1, NTH> s;
+    __device__ __forceinline__ void init(const dr_sim_state& st, const float* belief0, int pt0) { initState<NOPP + 1, NTH>(s, st, belief0, pt0); }
+    __device__ __forceinline__ void store(float* r, int tOrigin, float decay) const
+    {
+        if ((threadIdx.x & 31) == 0)
+            storeRec<NOPP + 1, NTH>(r, s, tOrigin, decay);
+    }
+    __device__ __forceinline__ void load(const float* r, int& tOrigin, float& decay) { loadRec<NOPP + 1, NTH>(r, s, tOrigin, decay); }
+    __device__ __forceinline__ GOut step(int t, int th, const Track& tr, const EnvParams& E, float u0, float u1, float minConf, bool& br)
+    {
+        return gstep<NOPP, NTH>(t, th, tr, E, cst(u0), cst(u1), s, minConf, br);
+    }
+};
+
+template <int NTH> struct ValueRollout<1, NTH>
+{
+    LaneState<NTH> s;
+    __device__ __forceinline__ void init(const dr_sim_state& st, const float* belief0, int pt0) { initLanes<NTH>(s, st, belief0, pt0); }
+    __device__ __forceinline__ void store(float* r, int tOrigin, float decay) const { storeLanes<NTH>(r, s, tOrigin, decay); }
+    __device__ __forceinline__ void load(const float* r, int& tOrigin, float& decay) { loadLanes<NTH>(r, s, tOrigin, decay); }
+    __device__ __forceinline__ GOut step(int t, int th, const Track& tr, const EnvParams& E, float u0, float u1, float minConf, bool& br)
+    {
+        return gstepLanes<NTH>(t, th, tr, E, u0, u1, s, minConf, br);
+    }
+};
+
 __device__ __forceinline__ float blockMaxAbs(const float* v, int n, float* red)
 {
     float m = 0.0f;
@@ -197,6 +228,7 @@ template <int NOPP, int NTH, bool SPL> __global__ void __launch_bounds__(GW * 32
 {
     constexpr int NA = NOPP + 1, NBP = NTH + 1;
     constexpr int NX = XState<NA, NTH>::NX, RW = recWords<NA, NTH>(), JW = NX + 1;
+    using Values = ValueRollout<NOPP, NTH>;
     static_assert(NX + 2 <= 32, "one lane per step input");
     extern __shared__ __align__(16) unsigned char smraw[];
     cg::cluster_group cluster = cg::this_cluster();
@@ -223,7 +255,8 @@ template <int NOPP, int NTH, bool SPL> __global__ void __launch_bounds__(GW * 32
 
     for (int i = threadIdx.x; i < ENV_HOST_WORDS; i += blockDim.x)
         ((float*)sE)[i] = ((const float*)&D.env)[i];
-    envDeviceTerms(*sE, D.env, threadIdx.x, blockDim.x);
+    __syncthreads();
+    envDeviceTerms(*sE, *sE, threadIdx.x, blockDim.x);
     for (int i = threadIdx.x; i < GRID_FLOATS; i += blockDim.x)
         sGrid[i] = D.grids[i];
     if constexpr (SPL)
@@ -274,20 +307,20 @@ template <int NOPP, int NTH, bool SPL> __global__ void __launch_bounds__(GW * 32
             int tau = 0;
             if (compatible)
             {
-                XState<NA, NTH> s;
-                initState<NA, NTH>(s, I.state, belief0, pt0);
+                Values s;
+                s.init(I.state, belief0, pt0);
                 float cost = 0.0f, decay = 1.0f;
                 int tOrigin = 0;
                 bool stop = false;
                 int t = 0;
                 for (; t < T && !stop; t++)
                 {
-                    if (lane == 0 && (C == 1 || t % C == 0))
-                        storeRec<NA, NTH>(sCk + (size_t)(C == 1 ? t : t / C) * RW, s, tOrigin, decay);
+                    if (C == 1 || t % C == 0)
+                        s.store(sCk + (size_t)(C == 1 ? t : t / C) * RW, tOrigin, decay);
                     float u0, u1;
-                    egoControl<SPL>(sU, sB, s.predTheta, t - tOrigin, M, T, u0, u1);
+                    egoControl<SPL>(sU, sB, s.s.predTheta, t - tOrigin, M, T, u0, u1);
                     bool br;
-                    const GOut o = gstep<NOPP, NTH>(t, th, tr, E, cst(u0), cst(u1), s, minConf, br);
+                    const GOut o = s.step(t, th, tr, E, u0, u1, minConf, br);
                     if (br)
                         tOrigin = t + 1;
                     stop = o.term != TERM_NONE;
@@ -300,10 +333,12 @@ template <int NOPP, int NTH, bool SPL> __global__ void __launch_bounds__(GW * 32
                     decay = __fmul_rn(decay, DECAY);
                 }
                 tau = t;
-                if (lane == 0)
-                    storeRec<NA, NTH>(sFin, s, tOrigin, decay);
+                s.store(sFin, tOrigin, decay);
+                __syncwarp();
+                XState<NA, NTH> last;
+                loadRec<NA, NTH>(sFin, last, tOrigin, decay);
                 float fe[N_WEIGHTS] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-                const Dv f = gfinal<NA, NTH>(s, E, w, fe);
+                const Dv f = gfinal<NA, NTH>(last, E, w, fe);
                 cost = __fadd_rn(cost, f.v);
                 feat[W_FINAL_ADV] = fe[W_FINAL_ADV];
                 feat[W_FINAL_OPP_ADV] = fe[W_FINAL_OPP_ADV];
@@ -351,20 +386,19 @@ template <int NOPP, int NTH, bool SPL> __global__ void __launch_bounds__(GW * 32
                 {
                     if (warp == 0)
                     {
-                        XState<NA, NTH> s;
+                        Values s;
                         int tO;
                         float dec;
-                        loadRec<NA, NTH>(sCk + (size_t)k * RW, s, tO, dec);
+                        s.load(sCk + (size_t)k * RW, tO, dec);
                         for (int t = t0; t < t1; t++)
                         {
-                            if (lane == 0)
-                                storeRec<NA, NTH>(sSeg + (size_t)(t - t0) * RW, s, tO, dec);
+                            s.store(sSeg + (size_t)(t - t0) * RW, tO, dec);
                             if (t + 1 == t1)
                                 break;
                             float u0, u1;
-                            egoControl<SPL>(sU, sB, s.predTheta, t - tO, M, T, u0, u1);
+                            egoControl<SPL>(sU, sB, s.s.predTheta, t - tO, M, T, u0, u1);
                             bool br;
-                            gstep<NOPP, NTH>(t, th, tr, E, cst(u0), cst(u1), s, minConf, br);
+                            s.step(t, th, tr, E, u0, u1, minConf, br);
                             if (br)
                                 tO = t + 1;
                             dec = __fmul_rn(dec, DECAY);

@@ -16,6 +16,7 @@
 // compiler removes it.
 #pragma once
 
+#include "../../include/drmppi.h"
 #include "model.cuh"
 
 namespace dr
@@ -305,28 +306,36 @@ __device__ __forceinline__ Dv gsample1(const float* __restrict__ arr, GPos q)
     return (1.0f - q.w) * arr[i0] + q.w * arr[i1];
 }
 
-// fastProjectOnTrack<false> (env_stratrace.h:88-162): nearest centreline sample in the
-// window around prevS (by value; first minimum in increasing index order), then the
-// nearest point of its two adjacent segments. Returns S, writes the signed lateral
-// distance.
-__device__ __forceinline__ Dv gproject(const Track& tr, float L, Dv px, Dv py, float prevS, Dv& lat)
+// fastProjectOnTrack<false> (env_stratrace.h:88-162): the nearest centreline sample in the
+// window around prevS (by value; first minimum in increasing index order), then the nearest
+// point of its two adjacent segments.
+//
+// The window's samples are spread over the warp: all 32 lanes take part with the same values
+// (only their tangents differ), lane j < 21 evaluates sample j, and the first of the lanes with
+// the least distance is the sample that a scan in increasing order keeps.
+__device__ __forceinline__ int gnearest(const Track& tr, float L, float px, float py, float prevS)
 {
     prevS = __fmul_rn(prevS, rcp(L));
     prevS = __fsub_rn(prevS, floorf(prevS));
-    const int idxPrev = (int)__fmul_rn(prevS, (float)NTS);
-    float best = INFINITY;
-    int bestJ = idxPrev - WIN;
-    for (int j = idxPrev - WIN; j <= idxPrev + WIN; j++)
+    const int j0 = (int)__fmul_rn(prevS, (float)NTS) - WIN;
+    const int lane = threadIdx.x & 31;
+    unsigned key = 0xffffffffu;
+    if (lane <= 2 * WIN)
     {
-        const float d0 = __fsub_rn(tr.p[j * 2 + 0], px.v), d1 = __fsub_rn(tr.p[j * 2 + 1], py.v);
+        const float d0 = __fsub_rn(tr.p[(j0 + lane) * 2 + 0], px), d1 = __fsub_rn(tr.p[(j0 + lane) * 2 + 1], py);
         const float sq = __fadd_rn(__fmul_rn(d0, d0), __fmul_rn(d1, d1));
-        if (sq < best)
-        {
-            best = sq;
-            bestJ = j;
-        }
+        if (sq < INFINITY) // like the scan, which starts from infinity; squares order as their words
+            key = __float_as_uint(sq);
     }
-    const int bestInd = wrapNts(bestJ + NTS); // bestJ >= -WIN
+    const unsigned least = __reduce_min_sync(0xffffffffu, key);
+    const int first = __ffs(__ballot_sync(0xffffffffu, key == least)) - 1;
+    return wrapNts(j0 + (least == 0xffffffffu ? 0 : first) + NTS); // j0 >= -WIN
+}
+
+// The nearest point of the two segments at sample bestInd. Returns S, writes the signed lateral
+// distance.
+__device__ __forceinline__ Dv gsegments(const Track& tr, float L, Dv px, Dv py, int bestInd, Dv& lat)
+{
     Dv bestSq = cst(INFINITY), bestS = cst(0.0f), cx = cst(0.0f), cy = cst(0.0f);
 #pragma unroll
     for (int seg = -1; seg <= 0; ++seg)
@@ -367,23 +376,28 @@ template <int NA> struct GGeo
     GPos tp[NA];
 };
 
+// of agent `a` (its place in g), from its arc length, lateral offset and velocity
+template <int NA>
+__device__ __forceinline__ void ggeometryOf(int a, const Track& tr, const EnvParams& E, Dv S, Dv lat, Dv v0, Dv v1, GGeo<NA>& g)
+{
+    g.tp[a] = gpos(S, E.trackLength);
+    Dv t0, t1;
+    gsample2(tr.t, g.tp[a], t0, t1);
+    const Dv inv = 1.0f / dsqrt(sq2(t0, t1));
+    g.tn0[a] = t0 * inv;
+    g.tn1[a] = t1 * inv;
+    g.kap[a] = gsample1(tr.k, g.tp[a]);
+    Dv metric = 1.0f - g.kap[a] * lat;
+    if (fabsf(metric.v) < 1e-12f)
+        metric = cst(copysignf(1e-12f, metric.v));
+    g.sdot[a] = (g.tn0[a] * v0 + g.tn1[a] * v1) / metric;
+}
+
 template <int NA, int NTH> __device__ __forceinline__ void ggeometry(const Track& tr, const EnvParams& E, const XState<NA, NTH>& s, GGeo<NA>& g)
 {
 #pragma unroll
     for (int a = 0; a < NA; a++)
-    {
-        g.tp[a] = gpos(s.S[a], E.trackLength);
-        Dv t0, t1;
-        gsample2(tr.t, g.tp[a], t0, t1);
-        const Dv inv = 1.0f / dsqrt(sq2(t0, t1));
-        g.tn0[a] = t0 * inv;
-        g.tn1[a] = t1 * inv;
-        g.kap[a] = gsample1(tr.k, g.tp[a]);
-        Dv metric = 1.0f - g.kap[a] * s.lat[a];
-        if (fabsf(metric.v) < 1e-12f)
-            metric = cst(copysignf(1e-12f, metric.v));
-        g.sdot[a] = (g.tn0[a] * s.vel[2 * a] + g.tn1[a] * s.vel[2 * a + 1]) / metric;
-    }
+        ggeometryOf<NA>(a, tr, E, s.S[a], s.lat[a], s.vel[2 * a], s.vel[2 * a + 1], g);
 }
 
 // Hypothesis-independent part of the opponent policy (env_stratrace.h:318-461, 611-706).
@@ -397,6 +411,31 @@ struct GOpp
     Dv tang0, tang1, norm0, norm1, kappa, e_n, v_t, v_n, metric_actual, a_centripetal, a_lat_max, distPos, distNeg;
     bool brakePos, brakeNeg;
 };
+
+// From the opponent's tangent and curvature and its offset and velocities in that frame (c.e_n,
+// c.v_t, c.v_n).
+__device__ __forceinline__ void goppFrame(int iOpp, const EnvParams& E, Dv tang0, Dv tang1, Dv kappa, GOpp& c)
+{
+    c.maxLatDis = __fsub_rn(E.trackWidth, __fmul_rn(E.droneRadius, E.maxOppLatDistFact));
+    c.maxAccel = E.maxAccel[iOpp];
+    c.maxAccelSq = __fmul_rn(c.maxAccel, c.maxAccel);
+    c.tang0 = tang0;
+    c.tang1 = tang1;
+    c.kappa = kappa;
+    c.norm0 = -c.tang1;
+    c.norm1 = c.tang0;
+    c.e_n_max = __fsub_rn(E.trackWidth, __fmul_rn(E.droneRadius, 1.2f));
+    Dv metric_actual = 1.0f - c.kappa * c.e_n;
+    if (fabsf(metric_actual.v) < 1e-6f)
+        metric_actual = cst(copysignf(1e-6f, metric_actual.v));
+    c.metric_actual = metric_actual;
+    c.a_centripetal = c.v_t * c.v_t * c.kappa / metric_actual;
+    c.a_lat_max = dmax(c.maxAccel - dabs(c.a_centripetal), cst(__fmul_rn(c.maxAccel, 0.2f)));
+    c.distPos = dmax(c.e_n_max - c.e_n, cst(0.001f));
+    c.distNeg = dmax(c.e_n_max + c.e_n, cst(0.001f));
+    c.brakePos = c.v_n.v > 0.0f && (c.v_n * c.v_n).v > (1.8f * c.a_lat_max * c.distPos).v;
+    c.brakeNeg = c.v_n.v < 0.0f && (c.v_n * c.v_n).v > (1.8f * c.a_lat_max * c.distNeg).v;
+}
 
 template <int NOPP, int NTH>
 __device__ __forceinline__ void goppCommon(int iOpp, const Track& tr, const EnvParams& E, const XState<NOPP + 1, NTH>& s, const GGeo<NOPP + 1>& g,
@@ -466,32 +505,15 @@ __device__ __forceinline__ void goppCommon(int iOpp, const Track& tr, const EnvP
         c.fasterThanJ[k] = c.sdot_i.v > sdj.v;
         c.oppLong[k] = vj0 * tj0 + vj1 * tj1;
     }
-    c.maxLatDis = __fsub_rn(E.trackWidth, __fmul_rn(E.droneRadius, E.maxOppLatDistFact));
-    c.maxAccel = E.maxAccel[iOpp];
-    c.maxAccelSq = __fmul_rn(c.maxAccel, c.maxAccel);
     Dv pc0, pc1;
     gsample2(tr.p, g.tp[iOpp], pc0, pc1);
-    c.tang0 = g.tn0[iOpp];
-    c.tang1 = g.tn1[iOpp];
-    c.kappa = g.kap[iOpp];
-    c.norm0 = -c.tang1;
-    c.norm1 = c.tang0;
+    const Dv tang0 = g.tn0[iOpp], tang1 = g.tn1[iOpp], norm0 = -tang1, norm1 = tang0;
     const Dv pos0 = s.pos[iOpp * 2], pos1 = s.pos[iOpp * 2 + 1];
     const Dv vel0 = s.vel[iOpp * 2], vel1 = s.vel[iOpp * 2 + 1];
-    c.e_n = (pos0 - pc0) * c.norm0 + (pos1 - pc1) * c.norm1;
-    c.v_t = vel0 * c.tang0 + vel1 * c.tang1;
-    c.v_n = vel0 * c.norm0 + vel1 * c.norm1;
-    c.e_n_max = __fsub_rn(E.trackWidth, __fmul_rn(E.droneRadius, 1.2f));
-    Dv metric_actual = 1.0f - c.kappa * c.e_n;
-    if (fabsf(metric_actual.v) < 1e-6f)
-        metric_actual = cst(copysignf(1e-6f, metric_actual.v));
-    c.metric_actual = metric_actual;
-    c.a_centripetal = c.v_t * c.v_t * c.kappa / metric_actual;
-    c.a_lat_max = dmax(c.maxAccel - dabs(c.a_centripetal), cst(__fmul_rn(c.maxAccel, 0.2f)));
-    c.distPos = dmax(c.e_n_max - c.e_n, cst(0.001f));
-    c.distNeg = dmax(c.e_n_max + c.e_n, cst(0.001f));
-    c.brakePos = c.v_n.v > 0.0f && (c.v_n * c.v_n).v > (1.8f * c.a_lat_max * c.distPos).v;
-    c.brakeNeg = c.v_n.v < 0.0f && (c.v_n * c.v_n).v > (1.8f * c.a_lat_max * c.distNeg).v;
+    c.e_n = (pos0 - pc0) * norm0 + (pos1 - pc1) * norm1;
+    c.v_t = vel0 * tang0 + vel1 * tang1;
+    c.v_n = vel0 * norm0 + vel1 * norm1;
+    goppFrame(iOpp, E, tang0, tang1, g.kap[iOpp], c);
 }
 
 // Hypothesis-dependent part: target lateral offset, speed goal and the resulting
@@ -656,7 +678,7 @@ __device__ __forceinline__ GOut gstep(int t, int trueTheta, const Track& tr, con
 #pragma unroll
     for (int a = 0; a < NA; a++)
     {
-        s.S[a] = gproject(tr, L, s.pos[2 * a], s.pos[2 * a + 1], Sint[a].v, s.lat[a]);
+        s.S[a] = gsegments(tr, L, s.pos[2 * a], s.pos[2 * a + 1], gnearest(tr, L, s.pos[2 * a].v, s.pos[2 * a + 1].v, Sint[a].v), s.lat[a]);
         if (s.S[a].v < __fsub_rn(prevS[a], __fmul_rn(L, 0.5f)))
             s.laps[a]++;
         if (s.S[a].v > __fadd_rn(prevS[a], __fmul_rn(L, 0.5f)))
@@ -734,6 +756,229 @@ __device__ __forceinline__ GOut gstep(int t, int trueTheta, const Track& tr, con
     r.bdRaw = bdRaw;
     r.oppWon = oppWon;
     r.winner = winner;
+    return r;
+}
+
+// The state of a value-only rollout with one opponent, over the lanes of a warp: even lanes hold
+// the ego, odd ones the opponent; the belief and the bookkeeping are alike on all.
+template <int NTH> struct LaneState
+{
+    float pos[2], vel[2], S, lat;
+    int laps;
+    float belief[NTH];
+    int predTheta, branchingTime;
+};
+
+template <int NTH> __device__ __forceinline__ void initLanes(LaneState<NTH>& s, const dr_sim_state& st, const float* belief0, int pt0)
+{
+    const int a = threadIdx.x & 1;
+    s.pos[0] = st.pos[2 * a];
+    s.pos[1] = st.pos[2 * a + 1];
+    s.vel[0] = st.vel[2 * a];
+    s.vel[1] = st.vel[2 * a + 1];
+    s.S = st.S[a];
+    s.lat = st.lat_dist[a];
+    s.laps = st.laps[a];
+#pragma unroll
+    for (int i = 0; i < NTH; i++)
+        s.belief[i] = belief0[i];
+    s.predTheta = pt0;
+    s.branchingTime = pt0 == 0 ? -1 : 0; // initBranchState (state.h:154-163)
+}
+
+// storeRec / loadRec of that state (lanes 0 and 1 write their agents)
+template <int NTH> __device__ __forceinline__ void storeLanes(float* r, const LaneState<NTH>& s, int tOrigin, float decay)
+{
+    constexpr int NX = XState<2, NTH>::NX;
+    const int lane = threadIdx.x & 31;
+    if (lane < 2)
+    {
+        r[2 * lane] = s.pos[0];
+        r[2 * lane + 1] = s.pos[1];
+        r[4 + 2 * lane] = s.vel[0];
+        r[4 + 2 * lane + 1] = s.vel[1];
+        r[8 + lane] = s.S;
+        r[10 + lane] = s.lat;
+        r[NX + lane] = __int_as_float(s.laps);
+    }
+    if (lane == 0)
+    {
+#pragma unroll
+        for (int i = 0; i < NTH; i++)
+            r[12 + i] = s.belief[i];
+        r[NX + 2] = __int_as_float(s.predTheta);
+        r[NX + 3] = __int_as_float(s.branchingTime);
+        r[NX + 4] = __int_as_float(tOrigin);
+        r[NX + 5] = decay;
+    }
+}
+
+template <int NTH> __device__ __forceinline__ void loadLanes(const float* r, LaneState<NTH>& s, int& tOrigin, float& decay)
+{
+    constexpr int NX = XState<2, NTH>::NX;
+    const int a = threadIdx.x & 1;
+    s.pos[0] = r[2 * a];
+    s.pos[1] = r[2 * a + 1];
+    s.vel[0] = r[4 + 2 * a];
+    s.vel[1] = r[4 + 2 * a + 1];
+    s.S = r[8 + a];
+    s.lat = r[10 + a];
+    s.laps = __float_as_int(r[NX + a]);
+#pragma unroll
+    for (int i = 0; i < NTH; i++)
+        s.belief[i] = r[12 + i];
+    s.predTheta = __float_as_int(r[NX + 2]);
+    s.branchingTime = __float_as_int(r[NX + 3]);
+    tOrigin = __float_as_int(r[NX + 4]);
+    decay = r[NX + 5];
+}
+
+// gstep's values with one opponent, by the 32 lanes of a warp: each agent's part on its lanes,
+// hypothesis h's policy and likelihood on lanes h, h + NTH, ..., the projection windows over all
+// of them. Every value is rounded explicitly, so the results are gstep's.
+template <int NTH>
+__device__ __forceinline__ GOut gstepLanes(int t, int trueTheta, const Track& tr, const EnvParams& E, float ego0, float ego1, LaneState<NTH>& s, float minConf,
+                                           bool& branched)
+{
+    constexpr unsigned ALL = 0xffffffffu;
+    const int role = threadIdx.x & 1, h = (threadIdx.x & 31) % NTH;
+    const float L = E.trackLength;
+    const float prevS = s.S;
+    auto of = [](float v, int lane) { return cst(__shfl_sync(ALL, v, lane)); };
+    GGeo<1> g;
+    const Dv p0 = cst(s.pos[0]), p1 = cst(s.pos[1]), v0 = cst(s.vel[0]), v1 = cst(s.vel[1]);
+    ggeometryOf<1>(0, tr, E, cst(s.S), cst(s.lat), v0, v1, g);
+    GOpp c;
+    {
+        Dv pc0, pc1;
+        gsample2(tr.p, g.tp[0], pc0, pc1);
+        const Dv norm0 = -g.tn1[0], norm1 = g.tn0[0];
+        const Dv e_n = (p0 - pc0) * norm0 + (p1 - pc1) * norm1;
+        const Dv along = v0 * g.tn0[0] + v1 * g.tn1[0];
+        const Dv v_n = v0 * norm0 + v1 * norm1;
+        const Dv S0 = of(s.S, 0), S1 = of(s.S, 1), lat0 = of(s.lat, 0), lat1 = of(s.lat, 1), sdot0 = of(g.sdot[0].v, 0), along0 = of(along.v, 0);
+        c.sdot_i = of(g.sdot[0].v, 1);
+        Dv dAhead = S0 - S1;
+        if (dAhead.v < 0.0f)
+            dAhead = dAhead + L;
+        Dv dBehind = S0 - S1;
+        if (dBehind.v > 0.0f)
+            dBehind = dBehind - L;
+#pragma unroll
+        for (int k = 0; k <= 1; k++)
+        {
+            const Dv deltaS = k ? dAhead : dBehind;
+            c.deltaS[k] = deltaS;
+            c.deltaE[k] = lat0 - lat1;
+            c.latJ[k] = lat0;
+            c.sdotJ[k] = sdot0;
+            c.blockTol[k] = __fmul_rn(E.maxSpeed[0], 0.3f);
+            c.shouldBlock[k] = (deltaS.v < 0.0f) && (deltaS.v > -L * 0.25f) && (__fadd_rn(sdot0.v, c.blockTol[k]) > c.sdot_i.v);
+            c.fasterThanJ[k] = c.sdot_i.v > sdot0.v;
+            c.oppLong[k] = along0;
+        }
+        c.e_n = of(e_n.v, 1);
+        c.v_t = of(along.v, 1);
+        c.v_n = of(v_n.v, 1);
+        goppFrame(1, E, of(g.tn0[0].v, 1), of(g.tn1[0].v, 1), of(g.kap[0].v, 1), c);
+    }
+    Dv n0, n1; // hypothesis h's action
+    goppAction(1, h, E, c, n0, n1);
+    const float o0 = __shfl_sync(ALL, n0.v, trueTheta), o1 = __shfl_sync(ALL, n1.v, trueTheta);
+    Dv act0 = cst(role ? o0 : ego0), act1 = cst(role ? o1 : ego1);
+    {
+        const Dv sq = sq2(act0, act1);
+        if (sq.v > __fmul_rn(E.maxAccel[role], E.maxAccel[role]))
+        {
+            const Dv f = E.maxAccel[role] / dsqrt(sq);
+            act0 *= f;
+            act1 *= f;
+        }
+    }
+    Dv q0 = p0, q1 = p1, w0 = v0, w1 = v1;
+    q0 += E.dt * v0;
+    q1 += E.dt * v1;
+    const Dv Sint = cst(s.S) + E.dt * g.sdot[0];
+    w0 += E.dt * act0;
+    w1 += E.dt * act1;
+    const Dv sqSpd = sq2(w0, w1);
+    if (sqSpd.v > __fmul_rn(E.maxSpeed[role], E.maxSpeed[role]))
+    {
+        const Dv sc = E.maxSpeed[role] / dsqrt(sqSpd);
+        w0 *= sc;
+        w1 *= sc;
+    }
+    const Dv pe0 = of(q0.v, 0), pe1 = of(q1.v, 0), po0 = of(q0.v, 1), po1 = of(q1.v, 1);
+    const int be = gnearest(tr, L, pe0.v, pe1.v, __shfl_sync(ALL, Sint.v, 0)), bo = gnearest(tr, L, po0.v, po1.v, __shfl_sync(ALL, Sint.v, 1));
+    Dv lat;
+    const Dv S = gsegments(tr, L, q0, q1, role ? bo : be, lat);
+    if (S.v < __fsub_rn(prevS, __fmul_rn(L, 0.5f)))
+        s.laps++;
+    if (S.v > __fadd_rn(prevS, __fmul_rn(L, 0.5f)))
+        s.laps--;
+    s.pos[0] = q0.v;
+    s.pos[1] = q1.v;
+    s.vel[0] = w0.v;
+    s.vel[1] = w1.v;
+    s.S = S.v;
+    s.lat = lat.v;
+    // belief update (env_stratrace.h:166-222)
+    {
+        const Dv a0 = of(act0.v, 1), a1 = of(act1.v, 1);
+        const Dv sqA = sq2(n0, n1);
+        Dv scale = cst(1.0f);
+        if (sqA.v > __fmul_rn(E.maxAccel[1], E.maxAccel[1]))
+            scale = E.maxAccel[1] / dsqrt(sqA);
+        const Dv sqDist = sq2(a0 - n0 * scale, a1 - n1 * scale);
+        const float sqSigma = beliefSqSigma(E.actionNoise[h][0]);
+        Dv ll = cst(0.0f);
+        ll = ll + ((-0.5f) * sqDist / sqSigma - logf(2.0f * M_PIf32) - E.logSqSigma[h][0]);
+        const Dv like = dexp(ll);
+        Dv sum = cst(0.0f);
+#pragma unroll
+        for (int i = 0; i < NTH; i++)
+        {
+            Dv b = cst(s.belief[i]);
+            b *= of(like.v, i);
+            s.belief[i] = b.v;
+            sum += b;
+        }
+        if (sum.v < 1e-20f)
+        {
+#pragma unroll
+            for (int i = 0; i < NTH; i++)
+                s.belief[i] = 1.0f / NTH;
+        }
+        else
+        {
+#pragma unroll
+            for (int i = 0; i < NTH; i++)
+                s.belief[i] = (cst(s.belief[i]) / sum).v;
+        }
+    }
+    // branching (findConfident, state.h:93-115)
+    int np = 0;
+#pragma unroll
+    for (int i = NTH - 1; i >= 0; i--)
+        if (s.belief[i] > minConf)
+            np = i + 1;
+    branched = false;
+    if (s.predTheta == 0 && np != 0)
+    {
+        s.predTheta = np;
+        s.branchingTime = t + 1;
+        branched = true;
+    }
+    // terminal tests (trackBoundaryDist / isOutside / isWinner, env_stratrace.h:226-274)
+    const float le = __shfl_sync(ALL, s.lat, 0), lo = __shfl_sync(ALL, s.lat, 1);
+    const int he = __shfl_sync(ALL, s.laps, 0), ho = __shfl_sync(ALL, s.laps, 1);
+    GOut r;
+    r.oppWon = ho >= E.nWinLaps;
+    const Dv minSq = dmin(cst(INFINITY), sq2(po0 - pe0, po1 - pe1));
+    r.bdRaw = dmin(dsqrt(minSq) - E.droneRadius, E.trackWidth - dabs(cst(le)));
+    r.winner = he >= E.nWinLaps || fabsf(lo) > __fsub_rn(E.trackWidth, E.droneRadius);
+    const float bdTerm = r.oppWon ? -1.0f : r.bdRaw.v;
+    r.term = bdTerm < E.droneRadius ? TERM_LOSE : r.winner ? TERM_WIN : TERM_NONE;
     return r;
 }
 
