@@ -378,23 +378,12 @@ struct dr_mppi_batch
         }
         CK(launchMppiPrologue(args(nullptr, 0, in), n, proSmem));
         // The previous plan's verification needs only the prologue's shifted plan and that
-        // plan's ego table, so it runs on a second stream while the rollout (a few warps per
+        // plan's ego table, so both run on a second stream while the rollout (a few warps per
         // SM) and the update run on the first; the new plan's verification follows the
-        // update. The previous plan's table is computed here, on the critical stream, before
-        // the fork: alone on the device it takes a few tens of microseconds, beside the
-        // rollout several times longer (its single warp per table row issues behind the
-        // rollout's warps), and the side verification could not start before it ends.
+        // update.
         bool side = verify && overlap && nVerOld > 0;
         if (side)
-        {
-            if (egoTable())
-            {
-                if (profile)
-                    timer->mark("ego_table_old", ex);
-                CK(launchEgo(ex, in, 1));
-            }
-            CK(cudaEventRecord(evFork, ex)); // the side verification depends on the prologue and the table
-        }
+            CK(cudaEventRecord(evFork, ex)); // the side stream's work depends on the prologue
         if (profile)
             timer->mark("rollout", ex);
         // the rollout is enqueued (captured) before the side verification, so that its
@@ -404,10 +393,15 @@ struct dr_mppi_batch
         {
             CK(cudaStreamWaitEvent(sideStream, evFork, 0));
             if (profile)
-            {
                 timerSide.begin();
-                timerSide.mark("verify_old", sideStream);
+            if (egoTable())
+            {
+                if (profile)
+                    timerSide.mark("ego_table_old", sideStream);
+                CK(launchEgo(sideStream, in, 1));
             }
+            if (profile)
+                timerSide.mark("verify_old", sideStream);
             CK(launchQueued(qargs(dVerOld, nVerOld, in, Q_VER_OLD, sidePerSm, sideStream), true));
             if (profile)
             {
