@@ -963,7 +963,7 @@ template <int NOPP, int NTH>
 __global__ void env_step_kernel(EnvParams Eh, const float* __restrict__ grids, int trueTheta, float a0, float a1, dr_sim_state* st, float* belief,
                                 int updateBelief, uint32_t k0, uint32_t k1, uint32_t step, int* term)
 {
-    __shared__ float sg[GRID_FLOATS];
+    __shared__ __align__(16) float sg[GRID_FLOATS];
     __shared__ EnvParams sE;
     for (int i = threadIdx.x; i < GRID_FLOATS; i += blockDim.x)
         sg[i] = grids[i];

@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(128) batch_env_step(const MppiDev* __restrict_
                                                       const float* __restrict__ actions, dr_sim_state* __restrict__ states, float* __restrict__ beliefs,
                                                       int updateBelief, uint32_t k0, uint32_t k1, int* __restrict__ terms)
 {
-    __shared__ float sg[GRID_FLOATS];
+    __shared__ __align__(16) float sg[GRID_FLOATS];
     __shared__ EnvParams sE;
     const int inst = blockIdx.x;
     const MppiDev& D = insts[inst];

@@ -89,6 +89,7 @@ constexpr int GRID_P = GRID_PAD * 2, GRID_T = GRID_ROW * 2, GRID_K = GRID_T + (N
 constexpr int GRID_PX = GRID_K + NTS + 1 + 1 + GRID_PAD, GRID_PY = GRID_PX + GRID_ROW;
 constexpr int GRID_CERT = GRID_PY - GRID_PAD + GRID_ROW;
 constexpr int GRID_FLOATS = GRID_CERT + NTS;
+static_assert(GRID_P % 2 == 0 && GRID_T % 2 == 0, "float2 samples");
 static_assert(GRID_FLOATS % 4 == 0 && GRID_PX % 2 == 0 && GRID_PY % 2 == 0 && GRID_PAD > WIN + 1, "grid layout");
 
 enum Term
@@ -243,21 +244,23 @@ __device__ __forceinline__ Track trackIn(const float* grids)
 
 // ---- track sampling (env_stratrace.h:44-85) ------------------------------------------
 
+// The next sample needs no wrap: the grids hold one past the last (and what follows that has
+// weight zero when s / L rounds to 1). `arr` is 8-byte aligned (GRID_P, GRID_T). Each read
+// brings both axes: the reads of shared memory are what a step's issue slots go to next after its
+// arithmetic (verification of 4 x K 524288 samples 0.354 -> 0.344 ms, control step 792 -> 764 us).
 __device__ __forceinline__ void sampleAt2(const float* __restrict__ arr, TrackPos q, float& o0, float& o1)
 {
-    const int idx0 = q.i0;
-    const int idx1 = wrapNts(idx0 + 1);
+    const float2* __restrict__ a = reinterpret_cast<const float2*>(arr) + q.i0;
+    const float2 a0 = a[0], a1 = a[1];
     const float t = q.w;
-    o0 = (1.0f - t) * arr[idx0 * 2 + 0] + t * arr[idx1 * 2 + 0];
-    o1 = (1.0f - t) * arr[idx0 * 2 + 1] + t * arr[idx1 * 2 + 1];
+    o0 = (1.0f - t) * a0.x + t * a1.x;
+    o1 = (1.0f - t) * a0.y + t * a1.y;
 }
 
 __device__ __forceinline__ float sampleAt1(const float* __restrict__ arr, TrackPos q)
 {
-    const int idx0 = q.i0;
-    const int idx1 = wrapNts(idx0 + 1);
     const float t = q.w;
-    return (1.0f - t) * arr[idx0] + t * arr[idx1];
+    return (1.0f - t) * arr[q.i0] + t * arr[q.i0 + 1];
 }
 
 __device__ __forceinline__ float sqNorm(float x, float y)
@@ -322,8 +325,8 @@ __device__ __forceinline__ float projectSegments(const Track& tr, float L, float
 // packed window scans below (sub, mul, then fma).
 __device__ __forceinline__ float windowSqDist(const Track& tr, int j0, int k, float px, float py)
 {
-    const int j = j0 + k;
-    const float d0 = __fsub_rn(tr.px[j], px), d1 = __fsub_rn(tr.py[j], py);
+    const float2 p = reinterpret_cast<const float2*>(tr.p)[j0 + k];
+    const float d0 = __fsub_rn(p.x, px), d1 = __fsub_rn(p.y, py);
     return __fmaf_rn(d1, d1, __fmul_rn(d0, d0));
 }
 

@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(128) mppi_predict(const MppiDev* __restrict__ 
                                                     PredictOut out, int nInst)
 {
     constexpr int NA = NOPP + 1;
-    __shared__ float sg[GRID_FLOATS];
+    __shared__ __align__(16) float sg[GRID_FLOATS];
     __shared__ EnvParams sE;
     const int inst = blockIdx.x;
     if (inst >= nInst)
@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(128) pr_predict(const PrDev* __restrict__ inst
 {
     constexpr int NA = NOPP + 1;
     constexpr int ROWS = NTH + 1;
-    __shared__ float sg[GRID_FLOATS];
+    __shared__ __align__(16) float sg[GRID_FLOATS];
     __shared__ EnvParams sE;
     const int inst = blockIdx.x;
     if (inst >= nInst)
