@@ -63,7 +63,7 @@ __host__ __device__ inline GateSmem gateRolloutLayout(int nbp, int T, int M, boo
         off = ga16(off + (size_t)T * M * 4);
     L.vbuf = off;
     if (spl)
-        off = ga16(off + (size_t)M * 2 * GPAIRS * 4);
+        off = ga16(off + (size_t)((M + 3) & ~3) * 2 * GPAIRS * 4);
     L.red = off;
     off = ga16(off + GRB * 4);
     L.total = off;
@@ -172,18 +172,15 @@ __global__ void __launch_bounds__(GRB) gate_rollout(const MppiDev* __restrict__ 
                     U4 r = draw(k0, k1, (uint32_t)s, (uint32_t)(b * M + m), step, S_MPPI_EPS, 0);
                     float e0 = scaled_normal(sig0, r.x);
                     float e1 = scaled_normal(sig1, r.y);
-                    vbuf[(m * GPAIRS + pair) * 2 + 0] = sKn[(b * M + m) * 2 + 0] + e0;
-                    vbuf[(m * GPAIRS + pair) * 2 + 1] = sKn[(b * M + m) * 2 + 1] + e1;
+                    float* v = vbuf + ((m >> 2) * 2 * GPAIRS + pair * 2) * 4 + (m & 3);
+                    v[0] = sKn[(b * M + m) * 2 + 0] + e0;
+                    v[4] = sKn[(b * M + m) * 2 + 1] + e1;
                 }
                 curB = b;
             }
             __syncwarp(mask);
             // a lane evaluates one axis of the control
-            const float* Brow = sB + local * M;
-            float sum = 0.0f;
-            for (int m = 0; m < M; m++)
-                sum += Brow[m] * vbuf[m * 2 * GPAIRS + threadIdx.x];
-            pairBoth(mask, role, sum, ctl0, ctl1);
+            pairBoth(mask, role, splineSum(sB + local * M, vbuf, 2 * GPAIRS, threadIdx.x, M), ctl0, ctl1);
         }
         else
         {

@@ -36,6 +36,41 @@ template <class V> __device__ __forceinline__ void pairBoth(unsigned mask, int r
     opp = role ? v : o;
 }
 
+// sum_m Brow[m] v[m] in knot order, v this column's knots: four at a time, [m / 4][column][4]
+// (columns of `cols`). Brow is 16-byte aligned when M is a multiple of 4. A 4-byte read a knot
+// and axis took a tenth of a spline rollout's issue slots: control step of 24 uneven agents
+// 1483 -> 1457 us.
+__device__ __forceinline__ float splineSum(const float* Brow, const float* vbuf, int cols, int col, int M)
+{
+    const float4* v = reinterpret_cast<const float4*>(vbuf) + col;
+    float sum = 0.0f;
+    if ((M & 3) == 0)
+    {
+        const float4* B = reinterpret_cast<const float4*>(Brow);
+        for (int q = 0; q < M / 4; q++)
+        {
+            const float4 b = B[q], x = v[q * cols];
+            sum += b.x * x.x;
+            sum += b.y * x.y;
+            sum += b.z * x.z;
+            sum += b.w * x.w;
+        }
+    }
+    else
+        for (int m = 0; m < M; m += 4)
+        {
+            const float4 x = v[m / 4 * cols];
+            sum += Brow[m] * x.x;
+            if (m + 1 < M)
+                sum += Brow[m + 1] * x.y;
+            if (m + 2 < M)
+                sum += Brow[m + 2] * x.z;
+            if (m + 3 < M)
+                sum += Brow[m + 3] * x.w;
+        }
+    return sum;
+}
+
 // Normal j of the step's environment noise (EnvNoise's stream, addressed by index: the two
 // lanes of a pair take different normals of one stream).
 struct PairNoise

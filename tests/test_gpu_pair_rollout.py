@@ -58,3 +58,21 @@ def test_pair_rollout_matches_oracle(gpu, nth, spl, K, certain, noise):
     mean = (w * np.where(fin, ct, 0.0)).sum(0) / w.sum(0)
     np.testing.assert_allclose(costs[0], mean, rtol=1e-5)
     assert np.array_equal(costs[1:][fin], ct[fin]) or np.allclose(costs[1:][fin], ct[fin], rtol=1e-6)
+
+
+@pytest.mark.parametrize("M", [2, 3, 4, 5, 7, 8, 9])
+def test_spline_sums_of_any_knot_count(gpu, M):
+    """Knots are summed four at a time: counts that fill no, one and two groups, and remainders."""
+    sc = S.circle_race(agent=1, seed=3, K=130, T=31, use_splines=True, n_theta=2, n_verif=64)
+    sc.mppi = S.make_mppi(K=130, T=31, use_splines=True, M=M, n_verif_samples=64, verif_horizon=20)
+    belief = sc.belief()
+    ctl = mppi_ctl(sc, nominal=np.random.default_rng(M).normal(0, 1.0, (3, 31, 2)).astype(np.float32))
+    ct, costs = np.zeros((2, 130), np.float32), np.zeros((3, 130), np.float32)
+    bu, bt = np.zeros((2, 130), np.int32), np.zeros((2, 130), np.int32)
+    abi.check(abi.lib().dr_mppi_debug_rollout(ctl.handle, C.byref(sc.state), abi.fptr(belief), abi.fptr(ct), abi.iptr(bu), abi.iptr(bt), abi.fptr(costs)),
+              "debug_rollout")
+    oct_, obu, obt = O.mppi_rollout(sc, belief, ctl.knots().copy(), O.mppi_noise(sc, 0), O.spline_matrix(sc.mppi), 0, prec=32)
+    fin = np.isfinite(oct_)
+    assert np.array_equal(fin, np.isfinite(ct))
+    assert np.mean(np.abs(ct[fin] - oct_[fin]) <= 1e-5 * np.maximum(1.0, np.abs(oct_[fin]))) >= 0.97
+    assert np.mean((bu == obu) & (bt == obt)) >= 0.97
