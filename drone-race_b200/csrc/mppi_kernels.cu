@@ -1629,10 +1629,21 @@ size_t mppiVerifySmem(int nth, int T)
            ((size_t)T * (3 + CLEAR_GROUPS) + 4) * 4 + (size_t)T * 4;
 }
 
+// Lockstep where the batch asks for it, and always by lane pairs with eight hypotheses: warps that
+// drift apart fetch that long step's code again and again. Rollouts of two agents of K 3001 x T 61:
+// 0.644 ms without the barrier, 0.605 with it; of 24 of K 2048: 3.43 and 3.24; of one of K 64:
+// 0.424 and 0.425. With four it gains 4 % at K 65536 and loses up to 12 % at K 1000 with splines,
+// with fewer it loses up to 5 %: there the batch chooses.
+template <int NOPP, int NTH> constexpr bool rolloutLockstep()
+{
+    return NOPP == 1 && NTH >= 8;
+}
+
 template <int NOPP, int NTH, bool SPL> static cudaError_t launchRolloutS(const LaunchArgs& a, size_t smem)
 {
-    auto k = a.queue ? (a.lockstep ? mppi_rollout<NOPP, NTH, SPL, true, true> : mppi_rollout<NOPP, NTH, SPL, true, false>)
-                     : (a.lockstep ? mppi_rollout<NOPP, NTH, SPL, false, true> : mppi_rollout<NOPP, NTH, SPL, false, false>);
+    constexpr bool ALWAYS = rolloutLockstep<NOPP, NTH>();
+    auto k = a.queue ? (a.lockstep ? mppi_rollout<NOPP, NTH, SPL, true, true> : mppi_rollout<NOPP, NTH, SPL, true, ALWAYS>)
+                     : (a.lockstep ? mppi_rollout<NOPP, NTH, SPL, false, true> : mppi_rollout<NOPP, NTH, SPL, false, ALWAYS>);
     ensureSmem(k, smem);
     const int work = a.nTiles * rolloutParts<NOPP>();
     k<<<a.queue && a.grid < work ? a.grid : work, RB, smem, a.stream>>>(a.mppi, a.mppiIn, a.tiles, a.nTiles, a.queue);
@@ -1665,13 +1676,13 @@ template <int NOPP, int NTH> static int residentT(bool verify, bool spl, size_t 
     }
     else if (spl)
     {
-        ensureSmem(mppi_rollout<NOPP, NTH, true, true, false>, smem);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, mppi_rollout<NOPP, NTH, true, true, false>, RB, smem);
+        ensureSmem(mppi_rollout<NOPP, NTH, true, true, rolloutLockstep<NOPP, NTH>()>, smem);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, mppi_rollout<NOPP, NTH, true, true, rolloutLockstep<NOPP, NTH>()>, RB, smem);
     }
     else
     {
-        ensureSmem(mppi_rollout<NOPP, NTH, false, true, false>, smem);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, mppi_rollout<NOPP, NTH, false, true, false>, RB, smem);
+        ensureSmem(mppi_rollout<NOPP, NTH, false, true, rolloutLockstep<NOPP, NTH>()>, smem);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, mppi_rollout<NOPP, NTH, false, true, rolloutLockstep<NOPP, NTH>()>, RB, smem);
     }
     return n;
 }
