@@ -7,15 +7,15 @@
 namespace dr
 {
 
-// Steps between two clearance tests of a verification warp: a test costs about 60
-// instructions, a step about 700. Four agents of 2 x 2^17 x 40, three drawn mid-race states
-// (B200, 1965 MHz; the verification of the new plan): without the test 0.52 / 0.45 / 0.55 ms,
-// every step 0.36 / 0.27 / 0.08, every second 0.35 / 0.26 / 0.08, every fourth 0.35 / 0.25 /
-// 0.10.
-#ifndef DR_CLEAR_EVERY
-#define DR_CLEAR_EVERY 2
-#endif
-constexpr int CLEAR_EVERY = DR_CLEAR_EVERY;
+// The steps before which a verification warp takes the clearance test (at the first one its
+// tile has): a test costs up to 100 instructions, a step about 700. Control steps of four agents
+// of 2 x 2^17 samples x 40, three drawn mid-race states (B200, 1965 MHz), every step / second /
+// fourth: 680 673 670, 622 613 608, 401 400 412 us; the second besides the fourths gives the last
+// row its 400. In the gate race every second / fourth / eighth: 712 698 718, 710 685 687 us.
+__device__ __forceinline__ bool clearTime(int t)
+{
+    return t == 2 || (t > 0 && t % 4 == 0);
+}
 
 // The block's rho in shared memory, from each group's own distances to those of it and the
 // later ones; all threads of the CTA, synchronised before and after by the caller.
@@ -27,29 +27,56 @@ __device__ __forceinline__ void clearSuffix(float* block, int H)
             cb.rho[g * H + j] = fmaxf(cb.rho[g * H + j], cb.rho[(g + 1) * H + j]);
 }
 
+// Whether opponents within (dp, dv) of position c and velocity w before step t (1-norms, which
+// bound the Euclidean ones) are out of reach of the ego after step j. The ego is within rho[j]
+// of the trajectory with no branch, xy[j].
+//
+// An opponent moves by its velocity before the step; then an acceleration clamped to amax is
+// added to that, and the result capped to vmax: a projection onto a ball that holds the old
+// velocity, which moves the new one neither farther from the old one nor, along any direction,
+// above vmax. So along the unit vector n its k = j - t + 1 steps take it at most
+// sum_i dt min(w n + dv + amax dt i, vmax), and with the first m of the minima taken on the left
+// and the others on the right, for any m, at most
+//   k dt w n + m dt dv + amax dt^2 m (m - 1) / 2 + (k - m) dt (vmax - w n).
+// n points to the ego from where the opponent gets at velocity w, m is about the steps that it
+// takes to reach vmax along n: of an opponent that follows the ego near its speed limit, the
+// limit bounds the way better than the acceleration does (control step of four agents with one
+// such follower 764 -> 667 us). Slack for the arithmetic (the
+// verification's approximate factors are within 1e-5, positions round to 2^-24 a step): two
+// millimetres, 1e-4 of the reach and of the speed limit's way, and a few H roundings of the
+// coordinates.
+__device__ __forceinline__ bool clearAfter(float dt, float radius, const float* xy, const float* rho, int H, int t, int j, float cx, float cy, float wx,
+                                           float wy, float dp, float dv, float vmax, float amax)
+{
+    const float k = (float)(j - t + 1), kd = k * dt;
+    const float ex = xy[2 * j] - (cx + kd * wx), ey = xy[2 * j + 1] - (cy + kd * wy);
+    const float sq = ex * ex + ey * ey;
+    const float room = fmaxf(vmax - (wx * ex + wy * ey) * rsqrtf(sq), 0.0f);
+    const float m = fmaxf(fminf(rintf(__fdividef(room - dv, amax * dt)), k), 0.0f);
+    const float way = kd * vmax;
+    const float reach = 2.0f * radius + rho[j] + dp + m * dt * dv + 0.5f * amax * dt * dt * (m * (m - 1.0f)) + (k - m) * dt * room;
+    const float slack = 2e-3f + 1e-4f * (reach + way) + 4.8e-7f * (float)H * (fabsf(cx) + fabsf(cy) + way);
+    const float need = reach + slack;
+    return sq > need * need && sq < 1e30f;
+}
+
 // Whether no remaining step (t .. H - 1) of the warp's active samples can bring an opponent
 // within two drone radii of the ego, or the ego off the track: then none of them can fail any
 // more (a sample fails at the first step with boundary distance below the drone radius) and
-// their remaining steps decide nothing. px .. vy: this lane's opponent before step t; xy: the
-// ego's trajectory with no branch (which stays on the track), rho: how far the samples' own may
-// be from it, after each step.
-//
-// An opponent whose speed is within its limit vmax moves k dt v in k steps plus at most
-// amax dt^2 k (k - 1) / 2: the step moves it by its velocity before the step and then adds an
-// acceleration clamped to amax, and the cap to vmax, a projection onto a ball that holds the
-// old velocity, never moves the new one farther from it. The warp's opponents lie within
-// (dp, dv) of the first active lane's in position and velocity (1-norms, which bound the
-// Euclidean ones). The ego is on a row of its table: within rho of the trajectory with no
-// branch. So after step j the two are at least |ego_j - (p + k dt v)| - rho - dp - k dt dv -
-// amax dt^2 k (k - 1) / 2 apart, k = j - t + 1. Slack for the arithmetic (the verification's
-// approximate factors are within 1e-5, positions round to 2^-24 a step): two millimetres, 1e-4
-// of the reach and of the speed limit's way, and a few H roundings of the coordinates.
+// their remaining steps decide nothing. px .. vy: this lane's opponent before step t; xy, rho:
+// the ego's trajectory with no branch (which stays on the track) and how far the samples' own
+// may be from it, after each step. witness: the last step that was within reach, -1 at first.
+// While a sample by itself can still be there, the others need no test: that takes 25
+// instructions in place of up to 100.
 __device__ __forceinline__ bool clearOfEgo(float dt, float radius, const float* xy, const float* rho, int H, int t, bool active, float px, float py,
-                                           float vx, float vy, float vmax, float amax)
+                                           float vx, float vy, float vmax, float amax, int& witness)
 {
     vmax = fabsf(vmax);
     amax = fabsf(amax);
     constexpr unsigned ALL = 0xffffffffu;
+    // the step that the last test found within reach: as long as a sample by itself can be there
+    if (witness >= t && __any_sync(ALL, active && !clearAfter(dt, radius, xy, rho, H, t, witness, px, py, vx, vy, 0.0f, 0.0f, vmax, amax)))
+        return false;
     const int lane = threadIdx.x & 31;
     const int src = __ffs(__ballot_sync(ALL, active)) - 1;
     const float cx = __shfl_sync(ALL, px, src), cy = __shfl_sync(ALL, py, src), wx = __shfl_sync(ALL, vx, src), wy = __shfl_sync(ALL, vy, src);
@@ -64,17 +91,28 @@ __device__ __forceinline__ bool clearOfEgo(float dt, float radius, const float* 
     // non-negative floats (and NaN, above them all) order as their words
     dp = __uint_as_float(__reduce_max_sync(ALL, __float_as_uint(dp)));
     dv = __uint_as_float(__reduce_max_sync(ALL, __float_as_uint(dv)));
-    for (int j = t + lane; j < H; j += 32)
+    if (!__all_sync(ALL, ok))
+        return false;
+    for (int j0 = H - 1 - (H - 1 - t) % 32; j0 >= t; j0 -= 32)
     {
-        const float k = (float)(j - t + 1), kd = k * dt;
-        const float ex = xy[2 * j] - (cx + kd * wx), ey = xy[2 * j + 1] - (cy + kd * wy);
-        const float way = kd * vmax;
-        const float reach = 2.0f * radius + rho[j] + dp + kd * dv + 0.5f * amax * dt * dt * (k * (k - 1.0f));
-        const float slack = 2e-3f + 1e-4f * (reach + way) + 4.8e-7f * (float)H * (fabsf(cx) + fabsf(cy) + way);
-        const float need = reach + slack;
-        ok = ok && ex * ex + ey * ey > need * need;
+        const int j = j0 + lane;
+        const unsigned near = __ballot_sync(ALL, j < H && !clearAfter(dt, radius, xy, rho, H, t, j, cx, cy, wx, wy, dp, dv, vmax, amax));
+        if (near)
+        {
+            witness = j0 + 31 - __clz(near);
+            return false;
+        }
     }
-    return __all_sync(ALL, ok);
+    return true;
+}
+
+// The same out of line: in line it costs the race's verification, at its 64 registers a thread,
+// 376 bytes of reloads against 82 (control steps of four agents 731 -> 677, 667 -> 613 us). The
+// gate race's step has the registers and is 3 % faster with the test in line.
+static __device__ __noinline__ bool clearOfEgoCall(float dt, float radius, const float* xy, const float* rho, int H, int t, bool active, float px, float py,
+                                                   float vx, float vy, float vmax, float amax, int& witness)
+{
+    return clearOfEgo(dt, radius, xy, rho, H, t, active, px, py, vx, vy, vmax, amax, witness);
 }
 
 } // namespace dr

@@ -418,10 +418,11 @@ __global__ void __launch_bounds__(VERIFY_TILE, (gateVerifyMinBlocks<NTH>())) gat
     if constexpr (CLEAR)
     {
         // every sample starts from the same state
+        int witness = -1;
         const ClearBlock<const float> cb(D.clear + (size_t)plan * clearWords(H), H);
         if (!dbgTheta && *cb.out == 0.0f &&
             clearOfEgo(D.gate->dt, D.gate->droneRadius, cb.xy, cb.all, H, 0, true, I.gstate.pos[2 * opp], I.gstate.pos[2 * opp + 1], I.gstate.vel[2 * opp],
-                       I.gstate.vel[2 * opp + 1], D.gate->maxSpeed[opp], D.gate->maxAccel[opp]))
+                       I.gstate.vel[2 * opp + 1], D.gate->maxSpeed[opp], D.gate->maxAccel[opp], witness))
             return;
     }
     if (threadIdx.x == 0)
@@ -502,14 +503,15 @@ __global__ void __launch_bounds__(VERIFY_TILE, (gateVerifyMinBlocks<NTH>())) gat
             else if (!__syncthreads_or(active))
                 break;
             if constexpr (CLEAR)
-                if (t % CLEAR_EVERY == 0)
+                if (clearTime(t))
                 {
+                    int witness = -1;
                     // the group of the earliest branch that a sample has taken or can take
                     const int tau = bs.predTheta == 0 || pt0 != 0 ? t : tOrigin - 1;
                     const int gr = __reduce_min_sync(0xffffffffu, active ? (unsigned)tau : ~0u) / (unsigned)clearPer(H);
                     const ClearBlock<const float> cb(sClear, H);
                     if (*cb.out == 0.0f && clearOfEgo(G.dt, G.droneRadius, cb.xy, cb.rho + gr * H, H, t, active, st.pos[2 * opp], st.pos[2 * opp + 1],
-                                                      st.vel[2 * opp], st.vel[2 * opp + 1], G.maxSpeed[opp], G.maxAccel[opp]))
+                                                      st.vel[2 * opp], st.vel[2 * opp + 1], G.maxSpeed[opp], G.maxAccel[opp], witness))
                         break;
                 }
             if (!active)

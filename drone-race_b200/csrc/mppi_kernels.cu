@@ -1435,8 +1435,11 @@ __global__ void __launch_bounds__(VERIFY_TILE, (verifyMinBlocks<NOPP, NTH>())) m
             const ClearBlock<const float> cb(D.clear + (size_t)plan * clearWords(H), H);
             clear = clear && *cb.out == 0.0f;
             for (int o = 1; o <= NOPP; o++)
-                clear = clear && clearOfEgo(D.env.dt, D.env.droneRadius, cb.xy, cb.all, H, 0, true, I.state.pos[2 * o], I.state.pos[2 * o + 1], I.state.vel[2 * o],
-                                            I.state.vel[2 * o + 1], D.env.maxSpeed[o], D.env.maxAccel[o]);
+            {
+                int witness = -1;
+                clear = clear && clearOfEgoCall(D.env.dt, D.env.droneRadius, cb.xy, cb.all, H, 0, true, I.state.pos[2 * o], I.state.pos[2 * o + 1], I.state.vel[2 * o],
+                                            I.state.vel[2 * o + 1], D.env.maxSpeed[o], D.env.maxAccel[o], witness);
+            }
             if (clear)
             {
                 if constexpr (PQ)
@@ -1527,6 +1530,10 @@ __global__ void __launch_bounds__(VERIFY_TILE, (verifyMinBlocks<NOPP, NTH>())) m
             using Noise = typename std::conditional<FAST, FastNoise, EnvNoise>::type;
             Noise rng(k0, k1, (uint32_t)v, (uint32_t)plan << 16, step, S_VERIF_ENV);
             int tOrigin = 0, t = 0, tEnd = H;
+            int witness[NOPP];
+#pragma unroll
+            for (int o = 0; o < NOPP; o++)
+                witness[o] = -1;
             bool failed = false;
             for (; t < H; t++)
             {
@@ -1535,7 +1542,7 @@ __global__ void __launch_bounds__(VERIFY_TILE, (verifyMinBlocks<NOPP, NTH>())) m
                 if (!__any_sync(0xffffffffu, active))
                     break;
                 if constexpr (EGO)
-                    if (t % CLEAR_EVERY == 0)
+                    if (clearTime(t))
                     {
                         // or once none of them can fail any more (see clearOfEgo)
                         // the group of the earliest branch that a sample has taken or can take
@@ -1545,8 +1552,8 @@ __global__ void __launch_bounds__(VERIFY_TILE, (verifyMinBlocks<NOPP, NTH>())) m
                         bool clear = *cb.out == 0.0f;
 #pragma unroll
                         for (int o = 1; o <= NOPP; o++)
-                            clear = clear && clearOfEgo(E.dt, E.droneRadius, cb.xy, cb.rho + gr * H, H, t, active, st.pos[2 * o], st.pos[2 * o + 1], st.vel[2 * o],
-                                                        st.vel[2 * o + 1], E.maxSpeed[o], E.maxAccel[o]);
+                            clear = clear && clearOfEgoCall(E.dt, E.droneRadius, cb.xy, cb.rho + gr * H, H, t, active, st.pos[2 * o], st.pos[2 * o + 1], st.vel[2 * o],
+                                                        st.vel[2 * o + 1], E.maxSpeed[o], E.maxAccel[o], witness[o - 1]);
                         if (clear)
                             break;
                     }

@@ -1,5 +1,5 @@
 """The fast verification stops stepping samples that can no longer collide (clearOfEgo in
-csrc/mppi_kernels.cu, from the ego tables of csrc/instance.cuh's clearance block). That changes
+csrc/clear.cuh, from the ego tables of csrc/instance.cuh's clearance block). That changes
 no result: per-sample failure times and counts equal, without tolerance, those of the
 verification that moves the ego in every sample and steps all of them to the end, over horizons
 around the table's step groups and over states from one in which nearly all samples collide to
@@ -54,6 +54,24 @@ def test_clearance_changes_no_failure(gpu, nth, H, gap, lat):
     sc, plan = _case(nth, H, gap, lat, seed=nth * 100 + H)
     for a, b in zip(_verify(sc, plan, True), _verify(sc, plan, False)):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("H", [5, 33, 64])
+@pytest.mark.parametrize("limit", [0.6, 0.99, 1.0])
+@pytest.mark.parametrize("gap", [-1.2, -1.6, -2.2])
+def test_clearance_of_followers_near_their_limit(gpu, H, limit, gap):
+    """An opponent behind the ego whose way the speed limit bounds before its acceleration does
+    (clearAfter), while the ego coasts or brakes."""
+    for brake in (0.0, 4.0):
+        sc, plan = _case(2, H, gap, 0.1, seed=H)
+        st = sc.state
+        v = limit * float(sc.env.max_speed[1])
+        n = float(np.hypot(st.vel[2], st.vel[3]))
+        st.vel[2], st.vel[3] = st.vel[2] * v / n * 0.9999, st.vel[3] * v / n * 0.9999
+        e = np.array([st.vel[0], st.vel[1]])
+        plan[:] = -brake * e / np.hypot(*e)
+        for a, b in zip(_verify(sc, plan, True), _verify(sc, plan, False)):
+            assert np.array_equal(a, b)
 
 
 def test_clear_tiles_of_whole_steps(gpu):
