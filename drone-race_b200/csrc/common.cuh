@@ -56,6 +56,15 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
                  : "memory");
 }
 
+// Orders this thread's ordinary accesses to shared memory before bulk copies that overwrite it: the
+// copies go through another proxy, which a CTA barrier does not order. Every thread that has
+// accessed memory that a later copy writes calls it, then takes the barrier behind which the copy is
+// issued.
+__device__ __forceinline__ void fence_before_bulk()
+{
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+
 // Default poll limit of a bounded wait (each poll is one try_wait, which may suspend the
 // thread for a short, hardware-defined time).
 constexpr int WAIT_POLLS = 1 << 22;

@@ -598,6 +598,8 @@ __global__ void __launch_bounds__(RB, (rolloutMinBlocks<NOPP, NTH>())) mppi_roll
             rolloutTilePair<NTH, SPL, LOCK>(D, I, tile, K, T, M, *sE, sGrid, sKn, sB, vbuf, red);
         else
             rolloutTile<NOPP, NTH, SPL, LOCK>(D, I, tile, K, T, M, *sE, sGrid, sKn, sB, vbuf, red);
+        if constexpr (PQ)
+            fence_before_bulk();
         __syncthreads(); // the next tile's staging and reduction buffer reuse shared memory
     }
 }
@@ -1199,6 +1201,8 @@ __global__ void __launch_bounds__(EGO_WARPS * 32) mppi_ego_table(const MppiDev* 
     constexpr unsigned ALL = 0xffffffffu;
     for (int plan = p0; plan <= p1; plan++)
     {
+        if (plan != p0)
+            fence_before_bulk(); // the clamp below wrote sPlan
         __syncthreads(); // the environment's terms, and the previous plan's rows are done with sPlan
         if (threadIdx.x == 0 && plan != p0)
         {
@@ -1601,6 +1605,8 @@ __global__ void __launch_bounds__(VERIFY_TILE, (verifyMinBlocks<NOPP, NTH>())) m
         for (int i = threadIdx.x; i < T; i += blockDim.x)
             if (hist[i])
                 atomicAdd(&D.fail[plan * T + i], hist[i]);
+        if constexpr (PQ)
+            fence_before_bulk();
         __syncthreads(); // the next tile's staging and histogram reuse shared memory
     }
 }
