@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(32) mppi_predict_pair(const MppiDev* __restric
     const int role = threadIdx.x & 1, th = (threadIdx.x >> 1) % NTH;
     const bool valid = threadIdx.x < 2 * NTH;
     const size_t row = (size_t)inst * NTH + th;
-    float2* pos = (float2*)(out.pos + row * out.tStride * 4) + role;
+    float* pos = out.pos + row * out.tStride * 4 + 2 * role; // the caller's: aligned as floats are
     float* act = out.act + row * out.tStride * 2;
     int* rec = out.rec + row * PREDICT_RECORD;
     const bool staged = __all_sync(ALL, mbar_wait(&bar, 0));
@@ -268,7 +268,8 @@ __global__ void __launch_bounds__(32) mppi_predict_pair(const MppiDev* __restric
         const StepOut o = pairStep<NTH, false, false>(mask, role, t, th, tr, E, e0, e1, 0.0f, 0.0f, s, bs, branched, D.cfg.minConf, PairNoise{});
         if (branched)
             tOrigin = t + 1;
-        pos[2 * t] = make_float2(s.pos[0], s.pos[1]);
+        pos[4 * t] = s.pos[0];
+        pos[4 * t + 1] = s.pos[1];
         act[2 * t + role] = role ? e1 : e0;
         cost += stateCost(o, E, D.cfg.w) * decay;
         decay *= DECAY;
@@ -287,7 +288,8 @@ __global__ void __launch_bounds__(32) mppi_predict_pair(const MppiDev* __restric
     // after a terminal step the engine repeats the last state and leaves the actions zero
     for (int u = staged ? (stopTime < 0 ? T : stopTime + 1) : 0; u < T; u++)
     {
-        pos[2 * u] = make_float2(s.pos[0], s.pos[1]);
+        pos[4 * u] = s.pos[0];
+        pos[4 * u + 1] = s.pos[1];
         act[2 * u + role] = 0.0f;
     }
     if (role != 0)
