@@ -188,10 +188,16 @@ __global__ void __launch_bounds__(128) mppi_predict(const MppiDev* __restrict__ 
 // mppi_predict with one opponent: a pair of lanes per hypothesis (pair_model.cuh), one warp a
 // controller, the track, the environment and the plan staged in shared memory. What bounds it is
 // the latency of its T dependent steps; a lane per agent halves their instructions, and the
-// plan no longer comes from global memory within them. A whole call (T 60, two hypotheses; B200,
-// 1965 MHz): 249 -> 181 us.
+// plan no longer comes from global memory within them. Four controllers (B200, 1965 MHz): T 60, two
+// hypotheses 227 -> 129 us, T 61, eight 525 -> 354; a whole host call of one, T 60: 269 -> 144.
+// The staging is plain loads, by PREDICT_THREADS threads of which one warp goes on: it waits for
+// nothing that could fail to arrive, and a prediction has no status to report that in. It takes the
+// time that a bulk copy took (129 / 131 us); one warp's loads take 6 us more, and without the bound
+// of one CTA an SM eight hypotheses get 105 registers a thread and take 373.
+constexpr int PREDICT_THREADS = 256;
+
 template <int NTH>
-__global__ void __launch_bounds__(32) mppi_predict_pair(const MppiDev* __restrict__ insts, const MppiIn* __restrict__ in,
+__global__ void __launch_bounds__(PREDICT_THREADS, 1) mppi_predict_pair(const MppiDev* __restrict__ insts, const MppiIn* __restrict__ in,
                                                         const dr_sim_state* __restrict__ states, const float* __restrict__ beliefs, int beliefStride,
                                                         PredictOut out, int nInst)
 {
@@ -199,7 +205,6 @@ __global__ void __launch_bounds__(32) mppi_predict_pair(const MppiDev* __restric
     __shared__ __align__(16) float sg[GRID_FLOATS];
     __shared__ __align__(16) float plan[(NTH + 1) * DR_MAX_T * 2];
     __shared__ EnvParams sE;
-    __shared__ __align__(8) uint64_t bar;
     constexpr unsigned ALL = 0xffffffffu;
     const int inst = blockIdx.x;
     if (inst >= nInst)
@@ -209,19 +214,18 @@ __global__ void __launch_bounds__(32) mppi_predict_pair(const MppiDev* __restric
     const int T = D.cfg.T, nbp = NTH + 1;
     // the controller's plan as the engine holds it: the chosen plan with the pending
     // warm-start shift of branch pendBranch (mppi_controller.cu:430-436)
-    const uint32_t planBytes = (uint32_t)(((size_t)nbp * T * 2 * 4 + 15) & ~(size_t)15);
-    if (threadIdx.x == 0)
-    {
-        mbar_init(&bar, 1);
-        mbar_expect_tx(&bar, GRID_FLOATS * 4 + planBytes);
-        bulk_g2s(sg, D.grids, GRID_FLOATS * 4, &bar);
-        bulk_g2s(plan, (I.pendBranch >= 0 && !I.pendUseNew) ? D.prevDense : D.dense, planBytes, &bar);
-    }
-    for (int i = threadIdx.x; i < ENV_HOST_WORDS; i += 32)
+    const float4* planFrom = (const float4*)((I.pendBranch >= 0 && !I.pendUseNew) ? D.prevDense : D.dense);
+    for (int i = threadIdx.x; i < GRID_FLOATS / 4; i += PREDICT_THREADS)
+        ((float4*)sg)[i] = ((const float4*)D.grids)[i];
+    for (int i = threadIdx.x; i < (nbp * T + 1) / 2; i += PREDICT_THREADS) // (the plans' storage is whole float4s)
+        ((float4*)plan)[i] = planFrom[i];
+    for (int i = threadIdx.x; i < ENV_HOST_WORDS; i += PREDICT_THREADS)
         ((float*)&sE)[i] = ((const float*)&D.env)[i];
-    __syncwarp();
-    envDeviceTerms(sE, sE, threadIdx.x, 32);
-    __syncwarp();
+    __syncthreads();
+    envDeviceTerms(sE, sE, threadIdx.x, PREDICT_THREADS);
+    __syncthreads();
+    if (threadIdx.x >= 32)
+        return;
     const int shiftB = (I.pendBranch >= 0 && I.pendBranch < nbp) ? I.pendBranch : -1;
     const int role = threadIdx.x & 1, th = (threadIdx.x >> 1) % NTH;
     const bool valid = threadIdx.x < 2 * NTH;
@@ -229,7 +233,6 @@ __global__ void __launch_bounds__(32) mppi_predict_pair(const MppiDev* __restric
     float* pos = out.pos + row * out.tStride * 4 + 2 * role; // the caller's: aligned as floats are
     float* act = out.act + row * out.tStride * 2;
     int* rec = out.rec + row * PREDICT_RECORD;
-    const bool staged = __all_sync(ALL, mbar_wait(&bar, 0));
     const EnvParams& E = sE;
     const Track tr = trackIn(sg);
     const dr_sim_state& st = states[inst];
@@ -253,7 +256,7 @@ __global__ void __launch_bounds__(32) mppi_predict_pair(const MppiDev* __restric
     bs.branchingTime = pred0 == 0 ? -1 : 0;
     float cost = 0.0f, decay = 1.0f;
     int tOrigin = 0, stopTime = -1, stopReason = EVT_TRUNCATED;
-    bool active = valid && staged; // (without the track: no prediction, like a plan that stops at once)
+    bool active = valid;
     for (int t = 0; t < T; t++)
     {
         const unsigned mask = __ballot_sync(ALL, active);
@@ -286,7 +289,7 @@ __global__ void __launch_bounds__(32) mppi_predict_pair(const MppiDev* __restric
     if (!valid)
         return;
     // after a terminal step the engine repeats the last state and leaves the actions zero
-    for (int u = staged ? (stopTime < 0 ? T : stopTime + 1) : 0; u < T; u++)
+    for (int u = stopTime < 0 ? T : stopTime + 1; u < T; u++)
     {
         pos[4 * u] = s.pos[0];
         pos[4 * u + 1] = s.pos[1];
@@ -386,10 +389,10 @@ cudaError_t launchMppiPredict(cudaStream_t stream, int nopp, int nth, const Mppi
 {
     switch (nopp * 16 + nth)
     {
-    case 1 * 16 + 1: mppi_predict_pair<1><<<nInst, 32, 0, stream>>>(insts, in, states, beliefs, beliefStride, out, nInst); break;
-    case 1 * 16 + 2: mppi_predict_pair<2><<<nInst, 32, 0, stream>>>(insts, in, states, beliefs, beliefStride, out, nInst); break;
-    case 1 * 16 + 4: mppi_predict_pair<4><<<nInst, 32, 0, stream>>>(insts, in, states, beliefs, beliefStride, out, nInst); break;
-    case 1 * 16 + 8: mppi_predict_pair<8><<<nInst, 32, 0, stream>>>(insts, in, states, beliefs, beliefStride, out, nInst); break;
+    case 1 * 16 + 1: mppi_predict_pair<1><<<nInst, PREDICT_THREADS, 0, stream>>>(insts, in, states, beliefs, beliefStride, out, nInst); break;
+    case 1 * 16 + 2: mppi_predict_pair<2><<<nInst, PREDICT_THREADS, 0, stream>>>(insts, in, states, beliefs, beliefStride, out, nInst); break;
+    case 1 * 16 + 4: mppi_predict_pair<4><<<nInst, PREDICT_THREADS, 0, stream>>>(insts, in, states, beliefs, beliefStride, out, nInst); break;
+    case 1 * 16 + 8: mppi_predict_pair<8><<<nInst, PREDICT_THREADS, 0, stream>>>(insts, in, states, beliefs, beliefStride, out, nInst); break;
     case 2 * 16 + 2: mppi_predict<2, 2><<<nInst, 128, 0, stream>>>(insts, in, states, beliefs, beliefStride, out, nInst); break;
     default: return cudaErrorInvalidValue;
     }

@@ -58,3 +58,15 @@ def test_a_kernel_that_stages_again_fences_first(kernel):
     body = next(b for _, k, b in LOOPS if k == kernel)
     fence = body.find("fence_before_bulk()")
     assert fence >= 0 and "__syncthreads()" in body[fence:], f"{kernel}: bulk copies over used shared memory without a proxy fence"
+
+
+WAITS = [(k, b) for _, k, b in kernels() if "mbar_wait" in b]
+
+
+@pytest.mark.parametrize("kernel", sorted({k for k, _ in WAITS}))
+def test_a_wait_that_runs_out_is_counted(kernel):
+    """A bounded wait that gives up leaves its kernel without its inputs: the count is how the host
+    learns of it (DR_ERR_TIMEOUT), so no kernel may go on without one."""
+    for k, body in WAITS:
+        if k == kernel:
+            assert re.search(r"!__syncthreads_and\(mbar_wait\([^;{]*\)\)\s*\{[^}]*atomicAdd\(&D\.stats\[1\], 1\);\s*return;", body), k
