@@ -25,8 +25,8 @@ struct MppiCfgDev
     int verify;
     int gradSteps; // gradient refinement steps (0: off)
     int sLo, sHi;  // this process's samples when the controller is sample-sharded (else 0, K)
-    // Bounded-wait test switch (dr_mppi_debug_stage_timeout): when set, the rollout and
-    // verification CTAs announce their staging bytes on the mbarrier but issue no copy, so
+    // Bounded-wait test switch (dr_mppi_debug_stage_timeout): when set, the rollout, ego table
+    // and verification CTAs announce their staging bytes on the mbarrier but issue no copy, so
     // the barrier's phase never completes and the wait gives up after waitPolls polls (0:
     // the default limit). Nothing is in flight when such a CTA returns.
     int dbgNoStage;

@@ -1186,8 +1186,11 @@ __global__ void __launch_bounds__(EGO_WARPS * 32) mppi_ego_table(const MppiDev* 
     {
         mbar_init(&bar, 1);
         mbar_expect_tx(&bar, GRID_FLOATS * 4 + planBytes);
-        bulk_g2s(sg, D.grids, GRID_FLOATS * 4, &bar);
-        bulk_g2s(sPlan, p0 == 0 ? D.dense : D.prevDense, planBytes, &bar);
+        if (!D.cfg.dbgNoStage)
+        {
+            bulk_g2s(sg, D.grids, GRID_FLOATS * 4, &bar);
+            bulk_g2s(sPlan, p0 == 0 ? D.dense : D.prevDense, planBytes, &bar);
+        }
     }
     copyEnv(&sE, &D.env);
     const EnvParams& E = sE;
@@ -1207,11 +1210,15 @@ __global__ void __launch_bounds__(EGO_WARPS * 32) mppi_ego_table(const MppiDev* 
         if (threadIdx.x == 0 && plan != p0)
         {
             mbar_expect_tx(&bar, planBytes);
-            bulk_g2s(sPlan, D.prevDense, planBytes, &bar);
+            if (!D.cfg.dbgNoStage)
+                bulk_g2s(sPlan, D.prevDense, planBytes, &bar);
         }
-        if (!__syncthreads_and(mbar_wait(&bar, (uint32_t)(plan - p0))))
+        if (!__syncthreads_and(mbar_wait(&bar, (uint32_t)(plan - p0), D.cfg.waitPolls)))
         {
-            // uniform: the step reports the timeout, as for the other kernels' staging
+            // uniform: the step reports the timeout, as for the other kernels' staging; a
+            // clearance block without its rows leaves no sample out
+            for (int q = plan + (int)threadIdx.x; q <= p1; q += blockDim.x)
+                *ClearBlock<float>(D.clear + (size_t)q * clearWords(H), H).out = 1.0f;
             if (threadIdx.x == 0)
                 atomicAdd(&D.stats[1], 1);
             return;

@@ -467,10 +467,10 @@ int dr_mppi_set_verify_exact(dr_mppi* h, int on);
  * reference. */
 int dr_mppi_set_ego_table(dr_mppi* h, int on);
 /* Test switch for the bounded device waits (no counterpart in the reference, whose
- * kernels have no device-side wait): while `on` is set, the rollout and verification CTAs
- * of this controller's own steps (dr_mppi_step, the dr_mppi_debug_* hooks) announce their
- * staging bytes but issue no copy, so each staging wait gives up after `polls` polls (<= 0:
- * the default limit) with nothing in flight; the step then returns DR_ERR_TIMEOUT and
+ * kernels have no device-side wait): while `on` is set, the rollout, ego table and
+ * verification CTAs of this controller's own steps (dr_mppi_step, the dr_mppi_debug_* hooks)
+ * announce their staging bytes but issue no copy, so each staging wait gives up after `polls`
+ * polls (<= 0: the default limit) with nothing in flight; the step then returns DR_ERR_TIMEOUT and
  * info->verif_timeouts counts the CTAs that gave up. Batches the controller joined later
  * keep their own copy of its settings. */
 int dr_mppi_debug_stage_timeout(dr_mppi* h, int on, int polls);
