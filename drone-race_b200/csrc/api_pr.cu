@@ -138,7 +138,8 @@ struct dr_prmppi_batch
     PrIn* hIn = nullptr;
     Tile *dRoll = nullptr, *dWa = nullptr;
     int nRoll = 0, nWa = 0;
-    int prThreads = PRS_TILE; // threads of a rollout CTA that shares egos (prTileThreads)
+    int prThreads = PRS_TILE; // threads of a rollout CTA that shares egos (sharedThreads)
+    int numSms = 0;
     size_t rollSmem = 0;
     bool useGraph = true;
     bool profiling = false;
@@ -173,6 +174,86 @@ struct dr_prmppi_batch
             if (h->env.action_noise_level != 0.0f || h->env.pos_noise_level != 0.0f || h->env.speed_noise_level != 0.0f)
                 return false;
         return true;
+    }
+
+    // the rollout moves a sample's ego once for all its hypotheses
+    bool rolloutShared() const
+    {
+        return nopp == 1 && egoShared() && slotsFor(prSlots) == 1;
+    }
+
+    static int tileSamples(const dr_prmppi* h, bool shared, int threads)
+    {
+        return h->envKind ? gatePrRolloutSamplesPerTile(shared, h->P, threads) : prRolloutSamplesPerTile(shared, h->P, threads);
+    }
+
+    long long countRollTiles(bool shared, int threads) const
+    {
+        long long n = 0;
+        for (auto* h : hs)
+        {
+            const int spb = tileSamples(h, shared, threads);
+            n += 2LL * ((h->sHi - h->sLo + spb - 1) / spb);
+        }
+        return n;
+    }
+
+    // Threads of a rollout CTA that shares egos: 512, two CTAs of which fill an SM, or fewer while
+    // the launch would leave SMs without one (one gate-race agent of 2 x 8 x 2048 samples: 74 CTAs
+    // of 512 threads or 148 of 256, 0.171 / 0.154 ms; B200, 1965 MHz).
+    int sharedThreads() const
+    {
+        int threads = PRS_TILE;
+        while (threads > PRS_MIN_TILE && countRollTiles(true, threads) < numSms)
+            threads /= 2;
+        return threads;
+    }
+
+    // Slots that a tile takes of a general kernel's CTA: whole warps, at least three, as few as leave
+    // the launch in the waves that full tiles take (one CTA an SM where those leave SMs without one).
+    // Tiles cut for the kernel that shares egos, which keeps room for them, left a part of the CTA
+    // idle: 4 agents with noise on the ego, P 1, K 16384 0.884 -> 0.640 ms, P 2, K 8192 0.899 ->
+    // 0.631; two opponents, P 2, K 8192 1.26 -> 0.92 (T 64; B200, 1965 MHz). Against full tiles: P 3,
+    // K 4096 0.621 -> 0.550; gate race, P 8, K 8192 0.529 -> 0.519; 2 slots a thread, P 8, K 2048
+    // 0.438 -> 0.420, K 512 0.431 -> 0.410 (with tiles of two warps 0.430).
+    int generalSlots() const
+    {
+        const long long full = countRollTiles(false, PRS_TILE);
+        const int wave = nopp == 1 && full > numSms ? 2 * numSms : numSms; // CTAs
+        const long long most = (full + wave - 1) / wave * wave;
+        int slots = 96;
+        while (slots < PRS_TILE && countRollTiles(false, slots) > most)
+            slots += 32;
+        return slots;
+    }
+
+    // the rollout's tile table, for the kernel that the batch's rollouts take
+    cudaError_t buildRollTiles()
+    {
+        const bool shared = rolloutShared();
+        const int threads = shared ? prThreads : generalSlots();
+        std::vector<Tile> roll;
+        for (int i = 0; i < (int)hs.size(); i++)
+        {
+            const dr_prmppi* h = hs[i];
+            const int spb = tileSamples(h, shared, threads);
+            for (int nr = 0; nr < 2; nr++)
+                for (int s0 = h->sLo; s0 < h->sHi; s0 += spb)
+                    roll.push_back(Tile{i, s0, std::min(spb, h->sHi - s0), nr});
+        }
+        Tile* d = nullptr;
+        cudaError_t e = cudaMalloc(&d, sizeof(Tile) * roll.size());
+        if (e == cudaSuccess)
+            e = cudaMemcpy(d, roll.data(), sizeof(Tile) * roll.size(), cudaMemcpyHostToDevice);
+        if (e != cudaSuccess)
+        {
+            cudaFree(d);
+            return e;
+        }
+        cudaFree(dRoll);
+        dRoll = d;
+        nRoll = (int)roll.size();
+        return cudaSuccess;
     }
 
     int maxSamples() const
@@ -413,26 +494,6 @@ struct dr_prmppi_batch
 namespace
 {
 
-// Threads of a rollout CTA that shares egos: 512, two CTAs of which fill an SM, or fewer while
-// the launch would leave SMs without one (one gate-race agent of 2 x 8 x 2048 samples: 74 CTAs
-// of 512 threads or 148 of 256, 0.171 / 0.154 ms; B200, 1965 MHz).
-int prTileThreads(dr_prmppi* const* hs, int n)
-{
-    int threads = PRS_TILE;
-    for (; threads > PRS_MIN_TILE; threads /= 2)
-    {
-        long long tiles = 0;
-        for (int i = 0; i < n; i++)
-        {
-            const int spb = hs[i]->envKind ? gatePrRolloutSamplesPerTile(hs[i]->P, threads) : prRolloutSamplesPerTile(hs[i]->P, threads);
-            tiles += 2LL * ((hs[i]->sHi - hs[i]->sLo + spb - 1) / spb);
-        }
-        if (tiles >= 148)
-            break;
-    }
-    return threads;
-}
-
 int buildPrBatch(dr_prmppi* const* hs, int n, cudaStream_t stream, bool ownStream, dr_prmppi_batch** out)
 {
     if (n <= 0 || !hs)
@@ -452,31 +513,26 @@ int buildPrBatch(dr_prmppi* const* hs, int n, cudaStream_t stream, bool ownStrea
     b->stream = stream;
     b->ownStream = ownStream;
     std::vector<PrDev> descs;
-    std::vector<Tile> roll, wa;
+    std::vector<Tile> wa;
+    CK(cudaDeviceGetAttribute(&b->numSms, cudaDevAttrMultiProcessorCount, b->device));
     if (b->nopp == 1 && b->egoShared())
-        b->prThreads = prTileThreads(hs, n);
+        b->prThreads = b->sharedThreads();
     for (int i = 0; i < n; i++)
     {
         dr_prmppi* h = hs[i];
         descs.push_back(h->desc);
-        const int spb = h->envKind ? gatePrRolloutSamplesPerTile(h->P, b->prThreads) : prRolloutSamplesPerTile(h->P, b->prThreads);
-        for (int nr = 0; nr < 2; nr++)
-            for (int s0 = h->sLo; s0 < h->sHi; s0 += spb)
-                roll.push_back(Tile{i, s0, std::min(spb, h->sHi - s0), nr});
         for (int w = 0; w < h->T; w++) // a step's three averages
             wa.push_back(Tile{i, w, 0, 0});
         b->maxT = std::max(b->maxT, h->T);
         b->maxP = std::max(b->maxP, h->P);
         b->rollSmem = std::max(b->rollSmem, h->envKind ? gatePrRolloutSmem(h->T, h->P) : prRolloutSmem(h->T, h->P));
     }
-    b->nRoll = (int)roll.size();
     b->nWa = (int)wa.size();
     CK(cudaMalloc(&b->dDesc, sizeof(PrDev) * n));
     CK(cudaMemcpy(b->dDesc, descs.data(), sizeof(PrDev) * n, cudaMemcpyHostToDevice));
     CK(cudaMalloc(&b->dIn, sizeof(PrIn) * n));
     CK(cudaMallocHost(&b->hIn, sizeof(PrIn) * n));
-    CK(cudaMalloc(&b->dRoll, sizeof(Tile) * roll.size()));
-    CK(cudaMemcpy(b->dRoll, roll.data(), sizeof(Tile) * roll.size(), cudaMemcpyHostToDevice));
+    CK(b->buildRollTiles());
     CK(cudaMalloc(&b->dWa, sizeof(Tile) * wa.size()));
     CK(cudaMemcpy(b->dWa, wa.data(), sizeof(Tile) * wa.size(), cudaMemcpyHostToDevice));
     *out = b.release();
@@ -1312,7 +1368,24 @@ extern "C" int dr_prmppi_batch_set_rollout_slots(dr_prmppi_batch* b, int slots)
     CK(cudaStreamSynchronize(b->stream));
     b->dropGraph();
     b->dropDevGraph();
+    const int before = b->prSlots;
+    const bool shared = b->rolloutShared();
     b->prSlots = slots;
+    if (b->rolloutShared() != shared)
+    {
+        const cudaError_t e = b->buildRollTiles();
+        if (e != cudaSuccess)
+            b->prSlots = before; // with the tiles that are there
+        CK(e);
+    }
+    return DR_OK;
+}
+
+extern "C" int dr_prmppi_batch_debug_rollout_tiles(const dr_prmppi_batch* b, int* tiles)
+{
+    if (!b || !tiles)
+        return fail(DR_ERR_INVALID_ARG, "NULL argument");
+    *tiles = b->nRoll;
     return DR_OK;
 }
 

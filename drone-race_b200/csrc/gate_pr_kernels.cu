@@ -665,9 +665,9 @@ size_t gatePrRolloutSmem(int T, int P)
     return a > b ? a : b;
 }
 
-int gatePrRolloutSamplesPerTile(int P, int threads)
+int gatePrRolloutSamplesPerTile(bool shared, int P, int threads)
 {
-    return gatePrSplit(P, threads).samples;
+    return prTileSamples(shared, P, threads, GPR_TILE);
 }
 
 template <int NTH, int ME> static cudaError_t gatePrRollT(const LaunchArgs& a, size_t smem)

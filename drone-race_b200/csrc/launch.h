@@ -125,7 +125,7 @@ cudaError_t launchGradNominal(cudaStream_t stream, const GradJob* jobs, int nJob
 
 // PR-MPPI on the gate race (gate_pr_kernels.cu); prologue and weighted averages are shared
 size_t gatePrRolloutSmem(int T, int P);
-int gatePrRolloutSamplesPerTile(int P, int threads);
+int gatePrRolloutSamplesPerTile(bool shared, int P, int threads);
 cudaError_t launchGatePrRollout(const LaunchArgs& a, int nth, int me, size_t smem);
 cudaError_t launchGatePrCandidates(const LaunchArgs& a, int nth, int me, int nInst, int maxT, int maxP);
 
@@ -169,7 +169,8 @@ cudaError_t launchCp(cudaStream_t stream, const uint32_t* k, int n, uint32_t N, 
 cudaError_t launchTrackGrids(cudaStream_t stream, const double* q, int nTracks, float* out, float* lengths);
 
 bool prSupported(int nopp, int nth);
-int prRolloutSamplesPerTile(int P, int threads);
+// threads: the CTA's where the kernel shares egos, else how many of its slots a tile takes
+int prRolloutSamplesPerTile(bool shared, int P, int threads);
 size_t prRolloutSmem(int T, int P);
 cudaError_t launchPrPrologue(const LaunchArgs& a, int nInst);
 cudaError_t launchPrRollout(const LaunchArgs& a, int nopp, int nth, size_t smem);

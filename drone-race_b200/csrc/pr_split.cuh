@@ -6,7 +6,7 @@
 namespace dr
 {
 
-constexpr int PRS_TILE = 512;     // threads of a CTA, unless the launch is small (prTileThreads)
+constexpr int PRS_TILE = 512;     // threads of a CTA, unless the launch is small (sharedThreads)
 #ifndef DR_PRS_MIN_TILE
 #define DR_PRS_MIN_TILE 128
 #endif
@@ -30,6 +30,13 @@ __host__ __device__ inline PrSplit prSplit(int P, int threads, int most)
     while (n > 1 && prWarps(n * P) + prWarps(n) > threads)
         n--;
     return PrSplit{n, prWarps(n * P)};
+}
+
+// The samples of a rollout tile: where the kernel shares egos, those whose opponents and egos fit
+// `threads` threads, else those whose (sample, hypothesis) slots do; `most` slots a CTA.
+__host__ __device__ inline int prTileSamples(bool shared, int P, int threads, int most)
+{
+    return shared ? prSplit(P, threads, most / P).samples : (threads < most ? threads : most) / P;
 }
 
 } // namespace dr

@@ -1177,9 +1177,9 @@ bool prSupported(int nopp, int nth)
     return key == 17 || key == 18 || key == 20 || key == 24 || key == 34;
 }
 
-int prRolloutSamplesPerTile(int P, int threads)
+int prRolloutSamplesPerTile(bool shared, int P, int threads)
 {
-    return prSplitOf(P, threads).samples;
+    return prTileSamples(shared, P, threads, PR_ROLL_TILE);
 }
 
 size_t prRolloutSmem(int T, int P)

@@ -506,6 +506,8 @@ int dr_prmppi_batch_get_kernel_times(dr_prmppi_batch* b, const char** names, flo
 int dr_prmppi_batch_set_rollout_slots(dr_prmppi_batch* b, int slots);
 
 /* ---- PR-MPPI test hooks ---------------------------------------------------------- */
+/* CTAs of the batch's rollout launch (of its present slot count). */
+int dr_prmppi_batch_debug_rollout_tiles(const dr_prmppi_batch* b, int* tiles);
 /* noise[T][K][DR_DIM] (prmppi_kernels.cu:17) and thetas[P] (prmppi_kernels.cu:23-51) of the next step. */
 int dr_prmppi_debug_noise(dr_prmppi* h, const float* belief, float* noise, size_t n, int32_t* thetas);
 /* Rollout of the next step (prmppi_kernels.cu:55-130): cost_nom/cost_rob [P][K][2]
