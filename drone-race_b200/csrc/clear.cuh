@@ -11,7 +11,8 @@ namespace dr
 // tile has): a test costs up to 100 instructions, a step about 700. Control steps of four agents
 // of 2 x 2^17 samples x 40, three drawn mid-race states (B200, 1965 MHz), every step / second /
 // fourth: 680 673 670, 622 613 608, 401 400 412 us; the second besides the fourths gives the last
-// row its 400. In the gate race every second / fourth / eighth: 712 698 718, 710 685 687 us.
+// row its 400. (The gate race's, whose steps cost less, wait longer after a test that failed by
+// more: clearOfEgo's wait.)
 __device__ __forceinline__ bool clearTime(int t)
 {
     return t == 2 || (t > 0 && t % 4 == 0);
@@ -46,7 +47,7 @@ __device__ __forceinline__ void clearSuffix(float* block, int H)
 // millimetres, 1e-4 of the reach and of the speed limit's way, and a few H roundings of the
 // coordinates.
 __device__ __forceinline__ bool clearAfter(float dt, float radius, const float* xy, const float* rho, int H, int t, int j, float cx, float cy, float wx,
-                                           float wy, float dp, float dv, float vmax, float amax)
+                                           float wy, float dp, float dv, float vmax, float amax, float* margin = nullptr)
 {
     const float k = (float)(j - t + 1), kd = k * dt;
     const float ex = xy[2 * j] - (cx + kd * wx), ey = xy[2 * j + 1] - (cy + kd * wy);
@@ -57,6 +58,8 @@ __device__ __forceinline__ bool clearAfter(float dt, float radius, const float* 
     const float reach = 2.0f * radius + rho[j] + dp + m * dt * dv + 0.5f * amax * dt * dt * (m * (m - 1.0f)) + (k - m) * dt * room;
     const float slack = 2e-3f + 1e-4f * (reach + way) + 4.8e-7f * (float)H * (fabsf(cx) + fabsf(cy) + way);
     const float need = reach + slack;
+    if (margin) // negative: by how much it is missed
+        *margin = sqrtf(sq) - need;
     return sq > need * need && sq < 1e30f;
 }
 
@@ -68,8 +71,15 @@ __device__ __forceinline__ bool clearAfter(float dt, float radius, const float* 
 // may be from it, after each step. witness: the last step that was within reach, -1 at first.
 // While a sample by itself can still be there, the others need no test: that takes 25
 // instructions in place of up to 100.
+// wait: after a test that failed, how many steps it takes until the reach to the witness is shorter
+// by what was missing (each takes amax dt^2 k off it), 0 where no number was missing. Tests before
+// that seldom succeed; fewer or more steps are worse. Gate race (B200, 1965 MHz), a test every
+// fourth step / waiting for all of it / half / 1.4 times / twice: control step of four agents in the
+// benchmark's state, where nothing clears, 1.006 / 0.964 / 0.970 / 0.966 / 0.990 ms (0.959 without
+// tests or tables), in three drawn mid-race states 624 584 523 / 617 577 513 / 622 579 515 /
+// 635 593 513 / 710 641 533 us.
 __device__ __forceinline__ bool clearOfEgo(float dt, float radius, const float* xy, const float* rho, int H, int t, bool active, float px, float py,
-                                           float vx, float vy, float vmax, float amax, int& witness)
+                                           float vx, float vy, float vmax, float amax, int& witness, int* wait = nullptr)
 {
     vmax = fabsf(vmax);
     amax = fabsf(amax);
@@ -96,10 +106,17 @@ __device__ __forceinline__ bool clearOfEgo(float dt, float radius, const float* 
     for (int j0 = H - 1 - (H - 1 - t) % 32; j0 >= t; j0 -= 32)
     {
         const int j = j0 + lane;
-        const unsigned near = __ballot_sync(ALL, j < H && !clearAfter(dt, radius, xy, rho, H, t, j, cx, cy, wx, wy, dp, dv, vmax, amax));
+        float margin = 0.0f;
+        const unsigned near = __ballot_sync(ALL, j < H && !clearAfter(dt, radius, xy, rho, H, t, j, cx, cy, wx, wy, dp, dv, vmax, amax, wait ? &margin : nullptr));
         if (near)
         {
-            witness = j0 + 31 - __clz(near);
+            const int last = 31 - __clz(near);
+            witness = j0 + last;
+            if (wait)
+            {
+                const float miss = -__shfl_sync(ALL, margin, last);
+                *wait = miss < 1e30f ? (int)fminf(__fdividef(miss, amax * dt * dt * (float)(witness - t + 1)), (float)H) : 0;
+            }
             return false;
         }
     }

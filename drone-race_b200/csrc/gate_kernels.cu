@@ -487,7 +487,7 @@ __global__ void __launch_bounds__(VERIFY_TILE, (gateVerifyMinBlocks<NTH>())) gat
         }
         using Noise = typename std::conditional<FAST, FastNoise, EnvNoise>::type;
         Noise rng(k0, k1, (uint32_t)v, (uint32_t)plan << 16, step, S_VERIF_ENV);
-        int tOrigin = 0, tEnd = H;
+        int tOrigin = 0, tEnd = H, next = 2;
         bool failed = false;
         for (int t = 0; t < H; t++)
         {
@@ -503,16 +503,17 @@ __global__ void __launch_bounds__(VERIFY_TILE, (gateVerifyMinBlocks<NTH>())) gat
             else if (!__syncthreads_or(active))
                 break;
             if constexpr (CLEAR)
-                if (clearTime(t))
+                if (t == next)
                 {
-                    int witness = -1;
+                    int witness = -1, wait = 0;
                     // the group of the earliest branch that a sample has taken or can take
                     const int tau = bs.predTheta == 0 || pt0 != 0 ? t : tOrigin - 1;
                     const int gr = __reduce_min_sync(0xffffffffu, active ? (unsigned)tau : ~0u) / (unsigned)clearPer(H);
                     const ClearBlock<const float> cb(sClear, H);
                     if (*cb.out == 0.0f && clearOfEgo(G.dt, G.droneRadius, cb.xy, cb.rho + gr * H, H, t, active, st.pos[2 * opp], st.pos[2 * opp + 1],
-                                                      st.vel[2 * opp], st.vel[2 * opp + 1], G.maxSpeed[opp], G.maxAccel[opp], witness))
+                                                      st.vel[2 * opp], st.vel[2 * opp + 1], G.maxSpeed[opp], G.maxAccel[opp], witness, &wait))
                         break;
+                    next = t + max(t == 2 ? 2 : 4, wait);
                 }
             if (!active)
                 continue;
