@@ -52,6 +52,29 @@ def _ensure_oracle():
 _ensure_oracle()
 
 
+# Tests against the reference's own build (its kernels, engine or host model). Where there is neither
+# that build nor a checkout to make it from they have nothing to compare with; where there is a
+# checkout, a build that failed fails them.
+NEEDS_REFERENCE = {
+    "test_reference_arm_line", "test_reference_engine_drives_mppi_dropin", "test_reference_engine_drives_prmppi_dropin",
+    "test_gate_rollout_matches_reference_kernel", "test_gate_update_matches_reference_kernels",
+    "test_gate_fast_verification_matches_reference_in_distribution", "test_gate_pr_rollout_matches_reference_kernel",
+    "test_gate_pr_step_matches_reference_kernels", "test_rollout_matches_reference_kernel", "test_update_matches_reference_kernels",
+    "test_headline_config_rollout_and_update_match_reference", "test_pr_update_and_candidates_match_reference",
+    "test_mppi_predictions_match_reference_engine", "test_mppi_prediction_branches_like_reference_host_model",
+    "test_prmppi_predictions_match_reference_engine", "test_pr_rollout_matches_reference_kernel", "test_env_step_matches_reference",
+    "test_fast_verification_matches_reference_in_distribution", "test_exact_verification_matches_reference_in_distribution",
+}
+
+
+def pytest_collection_modifyitems(items):
+    if O.REF_DIR.exists() or O.reference_dir().exists():
+        return
+    for item in items:
+        if getattr(item, "originalname", item.name) in NEEDS_REFERENCE:
+            item.add_marker(pytest.mark.skip(reason="reference build not present"))
+
+
 def has_gpu() -> bool:
     try:
         import torch
