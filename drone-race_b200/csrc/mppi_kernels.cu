@@ -1165,8 +1165,11 @@ __device__ __forceinline__ void egoAdvance(const EnvParams& E, const float* ctl,
     }
 }
 
+// The bound of five CTAs an SM gives it 96 registers a thread and no spills. Without one the compiler may
+// choose 80 with spills: beside the rollout the previous plan's table of four agents (H 40, two
+// hypotheses) then took 160 us in place of 19, and the control step 657 in place of 632.
 template <int NTH>
-__global__ void __launch_bounds__(EGO_WARPS * 32) mppi_ego_table(const MppiDev* __restrict__ insts, const MppiIn* __restrict__ in, int nInst, int plans)
+__global__ void __launch_bounds__(EGO_WARPS * 32, 5) mppi_ego_table(const MppiDev* __restrict__ insts, const MppiIn* __restrict__ in, int nInst, int plans)
 {
     __shared__ __align__(16) float sg[GRID_FLOATS];
     __shared__ __align__(16) float sPlan[(NTH + 1) * DR_MAX_T * 2];
