@@ -98,6 +98,9 @@ PR_FLOPS_PER_ROLLOUT_STEP = 411.7
 # launches fed by the device work queue, and with the shapes the autotuner picks.
 N_RACES = 256
 V_RACES = 4096
+# What the verification's steps are counted in: it does not step samples that provably can no longer
+# fail, from the start or from some step on, and how many that are depends on the state.
+VERIFY_UNITS = "sample-steps decided, whether stepped or proven unable to fail"
 WL = {"kind": "strat"}  # the workload of this run (set from --workload)
 
 
@@ -136,9 +139,9 @@ def _ref_variant(O) -> str:
 
 # DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) from one ncu capture
 # of each kernel on this workload (--quick --no-overlap, 3 steps); grids, plans and tile
-# tables stay in L2, so DRAM traffic is spilled registers and first-touch reads, about 0.9
-# MB per verification launch (both plans, with the ego tables).
-TRAFFIC_PER_LAUNCH: dict[str, float] = {"verify": 855040.0, "rollout": 168960.0}
+# tables stay in L2, so DRAM traffic is first-touch reads (and, in a verification that steps
+# its samples, which this state's first steps hardly do, spilled registers: about 0.9 MB).
+TRAFFIC_PER_LAUNCH: dict[str, float] = {"verify": 95232.0, "rollout": 140544.0}
 
 
 def _package():
@@ -609,10 +612,12 @@ def run_ours(args) -> None:
                 "peak_source": "FP32 FMA rate of 148 SMs x 128 lanes at the median SM clock sampled during the timed region (MEASURED_PEAKS.json has no FP32 figure)",
                 "units_per_launch": units[dom], "flops_per_unit": flops_unit[dom], "kernel_ms": kt_serial[dom],
                 "measured": f"CUDA events around each launch on its stream, {serial_steps} steps with both plans verified in one launch"}
-        step_flops = sum(units[k] * flops_unit[k] for k in units)
-        ach_step = step_flops / (ms_per_step / 1e3) / 1e12
+        if dom == "verify":
+            roof["units"] = VERIFY_UNITS + ": an upper bound of what the launch executes"
+        ach_step = units["rollout"] * flops_unit["rollout"] / (ms_per_step / 1e3) / 1e12
         roof_step = {"bound": "fp32", "achieved": ach_step, "peak": peak, "unit": "TFLOP/s", "frac": ach_step / peak,
-                     "scope": "all FP32 work of one control step (rollout + both verifications) / device step time of the timed region"}
+                     "scope": "the rollout's FP32 work / device step time of the timed region: a lower bound of a step's work, without the "
+                              "verification's " + VERIFY_UNITS}
 
     cpu = None
     if rank == 0 and world == 1 and not args.no_cpu_baseline and not args.quick:
@@ -638,6 +643,7 @@ def run_ours(args) -> None:
                    "l2": "working set per step < L2; steps are dependent control steps of the same controllers"},
         "rollout_steps_per_s": world * rollout_steps * args.steps / (ms / 1e3),
         "verify_steps_per_s": world * AGENTS * 2 * V * VERIF_H * args.steps / (ms / 1e3),
+        "verify_steps": VERIFY_UNITS,
         "kernel_ms": kt,
         "kernel_timeline_ms": timeline,
         "kernel_ms_serial": kt_serial,
@@ -1023,7 +1029,6 @@ def run_ours_races(args) -> None:
         e2e = {"value": world * n_agents * e2e_steps / e2e_s, "unit": "agent control steps/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                "ms_per_step": e2e_s / e2e_steps * 1e3}
     rollout_units = sum(s.mppi.n_samples * N_THETA * s.mppi.n_timesteps for s in scs)
-    verify_units = sum(2 * V_RACES * min(40, s.mppi.n_timesteps) for s in scs)
     kt_sum = {}
     for kt in kts:
         for k, v in kt.items():
@@ -1031,9 +1036,10 @@ def run_ours_races(args) -> None:
     roof = None
     if clk.get("sm_mhz"):
         peak = 2 * 128 * 148 * clk["sm_mhz"] * 1e6 / 1e12
-        ach = (rollout_units * FLOPS_PER_ROLLOUT_STEP + verify_units * FLOPS_PER_VERIFY_STEP) / (ms_per_step / 1e3) / 1e12
+        ach = rollout_units * FLOPS_PER_ROLLOUT_STEP / (ms_per_step / 1e3) / 1e12
         roof = {"bound": "fp32", "achieved": ach, "peak": peak, "unit": "TFLOP/s", "frac": ach / peak, "traffic": None,
-                "scope": "all FP32 work of one control step of every agent (dense-control FLOP counts; spline evaluation not counted) / device step time",
+                "scope": "FP32 work of the rollouts of one control step of every agent (dense-control FLOP counts; spline evaluation not counted) / "
+                         "device step time: a lower bound of a step's work, without the verification's " + VERIFY_UNITS,
                 "peak_source": "FP32 FMA rate of 148 SMs x 128 lanes at the median SM clock sampled during the timed region"}
     line = {
         "metric": "agent_control_steps_per_s",
@@ -1233,15 +1239,15 @@ def run_ours_mixed(args) -> None:
     mppi_scs = [s for s in scs if s.kind != "pr"]
     pr_scs = [s for s in scs if s.kind == "pr"]
     rollout_units = sum(s.mppi.n_samples * s.n_theta * s.mppi.n_timesteps for s in mppi_scs)
-    verify_units = sum(2 * V_RACES * min(40, s.mppi.n_timesteps) for s in mppi_scs)
     pr_units = sum(2 * s.prmppi.P * s.prmppi.n_samples * s.prmppi.n_timesteps for s in pr_scs)
     roof = None
     if clk.get("sm_mhz"):
         peak = 2 * 128 * 148 * clk["sm_mhz"] * 1e6 / 1e12
-        ach = (rollout_units * FLOPS_PER_ROLLOUT_STEP + verify_units * FLOPS_PER_VERIFY_STEP + pr_units * PR_FLOPS_PER_ROLLOUT_STEP) / (ms_per_step / 1e3) / 1e12
+        ach = (rollout_units * FLOPS_PER_ROLLOUT_STEP + pr_units * PR_FLOPS_PER_ROLLOUT_STEP) / (ms_per_step / 1e3) / 1e12
         roof = {"bound": "fp32", "achieved": ach, "peak": peak, "unit": "TFLOP/s", "frac": ach / peak, "traffic": None,
-                "scope": "FP32 work of the MPPI rollouts and verifications and the PR-MPPI rollouts of one control step of every agent (dense-control "
-                         "FLOP counts; spline evaluation, updates, gradient refinement and candidate re-checks not counted) / device step time",
+                "scope": "FP32 work of the MPPI and PR-MPPI rollouts of one control step of every agent (dense-control FLOP counts; spline evaluation, "
+                         "updates, gradient refinement and candidate re-checks not counted) / device step time: a lower bound of a step's work, "
+                         "without the verification's " + VERIFY_UNITS,
                 "peak_source": "FP32 FMA rate of 148 SMs x 128 lanes at the median SM clock sampled during the timed region"}
     kinds = {k: sum(1 for s in scs if s.kind == k) for k in ("plain", "grad", "pr")}
     line = {

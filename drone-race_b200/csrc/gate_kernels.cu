@@ -1,9 +1,10 @@
 // MPPI kernels of the gate race (the reference's kernels.cu compiled with
 // USE_ENV_DRONERACE): the rollout with per-branch cost aggregation and the plan
-// verification, built like mppi_rollout / mppi_verify (one thread per (sample,
-// hypothesis), resp. per verification sample; state in registers; racelines in shared
-// memory, staged by a bulk copy; gate parameters copied to shared memory; perturbations
-// from Philox) on the model of gate_model.cuh. The prologue and the update kernels of
+// verification, built like mppi_rollout / mppi_verify (a pair of lanes per (sample,
+// hypothesis), resp. a thread per verification sample; state in registers; racelines in
+// shared memory, staged by a bulk copy; gate parameters copied to shared memory;
+// perturbations from Philox) on the model of gate_model.cuh and gate_pair.cuh. The prologue
+// and the update kernels of
 // mppi_kernels.cu serve both environments (they see only costs, bookkeeping and plans).
 #include <cstdio>
 
@@ -374,8 +375,8 @@ __global__ void __launch_bounds__(GCLEAR) gate_clear(const MppiDev* __restrict__
 }
 
 // verifyNominalFailureKernel (kernels.cu:488-551) on the gate race:
-// environmentStep<true, true, false, false>; one thread per sample, both plans in one
-// grid, the CTA's warps in step (a barrier per step) as in mppi_verify.
+// environmentStep<true, true, false, false>; one thread per sample, each plan's tiles in
+// the grid, the CTA's warps in step (a barrier per step) in the exact flavour only.
 // Two 512-thread CTAs per SM (64 registers a thread, ~20 bytes spilled) for up to four
 // hypotheses: measured on the 4 x 2 x 2^17 x 40 gate verification (B200, 1965 MHz)
 // 2.66 ms against 3.42 ms with one CTA per SM (128 registers, no spills).

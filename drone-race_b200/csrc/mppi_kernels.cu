@@ -13,13 +13,17 @@
 //                   memory by bulk copies; the perturbation is drawn from Philox instead of
 //                   being read from a stored noise tensor.
 //   mppi_update     per (branch plan, knot): masked minimum, exponential weights and the
-//                   weighted average of the regenerated perturbations in one block
+//                   weighted average of the regenerated perturbations by one CTA or, with
+//                   many samples and few knots, a cluster of up to eight
 //                   (computeMaskedMinCostsKernel + weightedAverageKernelUnified,
 //                   kernels.cu:221-408; the sums are accumulated in the reference's
-//                   256-thread order); the last block of an instance to finish also does
+//                   256-lane order); the last one of an instance to finish also does
 //                   the spline interpolation and the clamp (kernels.cu:411-456).
+//   mppi_ego_table  the ego's moves under a plan, which the verification's samples share,
+//                   and its whereabouts (the clearance block).
 //   mppi_verify     Monte-Carlo failure counts of the new and the previous plan
-//                   (verifyNominalFailureKernel, kernels.cu:488-551), both plans in one grid.
+//                   (verifyNominalFailureKernel, kernels.cu:488-551), a launch a plan or
+//                   both in one grid; samples that can no longer fail are not stepped on.
 #include <cooperative_groups.h>
 
 #include <cfloat>
@@ -361,7 +365,8 @@ __device__ __forceinline__ void rolloutTile(const MppiDev& D, const MppiIn& I, c
 // issue and divergence (samples that end early leave their lanes idle) from there. Against a
 // thread per (sample, hypothesis), which moved both agents one after the other (B200, 1965
 // MHz): one agent of K 1024 x 2 x T 50 0.23 -> 0.15 ms, four agents of K 4096 x 2 x T 64
-// 0.32 -> 0.21 alone, one of K 65536 x 2 x T 80 with spline controls 1.45 -> 1.26.
+// 0.32 -> 0.22 alone, one of K 65536 x 2 x T 80 with spline controls, the previous plan's
+// verification beside it, 1.46 -> 1.09.
 template <int NTH, bool SPL, bool LOCK>
 __device__ __forceinline__ void rolloutTilePair(const MppiDev& D, const MppiIn& I, const Tile& tile, int K, int T, int M, const EnvParams& E,
                                                 const float* sGrid, const float* sKn, const float* sB, float* vbuf, float* red)

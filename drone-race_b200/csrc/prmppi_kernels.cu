@@ -8,7 +8,10 @@
 //                  nominal + Philox perturbation under theta_p with running and safety cost
 //                  (PRMPPIfullRolloutKernel, :55-130); the hypotheses of a sample sit in
 //                  neighbouring threads, so the per-sample average over p and the safety
-//                  indicator (PRMPPIcostAvgKernel, :134-166) are done in the epilogue.
+//                  indicator (PRMPPIcostAvgKernel, :134-166) are done in the epilogue. For
+//                  two opponents, noise on the ego or several slots a thread; otherwise
+//   pr_rollout_shared   the same with the ego of a sample moved once, by warps of its own
+//                  a step ahead of its opponents' (and pr_candidates_shared likewise).
 //   pr_weighted    per t, the three averages: minimum of the averaged cost (PRMPPIcomputeMinCosts-
 //                  Kernel, :169-199), exponential weights and the weighted average of the
 //                  absolute perturbed controls (PRMPPIWeightedAverageKernel, :204-282),

@@ -463,8 +463,9 @@ int dr_mppi_set_verify_exact(dr_mppi* h, int on);
  * built only when no environment noise moves the ego and both plans' tables fit in 16 MiB
  * (the library's build-time DR_EGO_TABLE_MAX_BYTES). With them comes the clearance block of
  * a plan (in the gate race the block alone), by which samples that can no longer collide are
- * not stepped on. The failure times are the same either way; off is slower. Set it before batching the controller. No counterpart in the
- * reference. */
+ * not stepped on. The failure times are the same either way; off is slower (in the gate race
+ * up to 1 % faster where no sample ever clears). Set it before batching the controller. No
+ * counterpart in the reference. */
 int dr_mppi_set_ego_table(dr_mppi* h, int on);
 /* Test switch for the bounded device waits (no counterpart in the reference, whose
  * kernels have no device-side wait): while `on` is set, the rollout, ego table and
@@ -502,7 +503,7 @@ int dr_prmppi_batch_get_kernel_times(dr_prmppi_batch* b, const char** names, flo
  * only where no environment noise moves the ego and P is a multiple of it (else 1).
  * Strategic race batches. No counterpart in the reference. With 1 the ego of a sample is
  * moved once for all its slots by a warp of its own, one step ahead of them; on the 4-agent
- * P 8 x K 2048 x H 64 workload that takes 0.24 - 0.34 ms, 2 / 4 slots a thread 0.61 / 1.02. */
+ * P 8 x K 2048 x H 64 workload that takes 0.34 ms, 2 / 4 slots a thread 0.56 / 0.90. */
 int dr_prmppi_batch_set_rollout_slots(dr_prmppi_batch* b, int slots);
 
 /* ---- PR-MPPI test hooks ---------------------------------------------------------- */
