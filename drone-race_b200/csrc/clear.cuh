@@ -52,14 +52,15 @@ __device__ __forceinline__ bool clearAfter(float dt, float radius, const float* 
     const float k = (float)(j - t + 1), kd = k * dt;
     const float ex = xy[2 * j] - (cx + kd * wx), ey = xy[2 * j + 1] - (cy + kd * wy);
     const float sq = ex * ex + ey * ey;
-    const float room = fmaxf(vmax - (wx * ex + wy * ey) * rsqrtf(sq), 0.0f);
+    const float inv = rsqrtf(sq);
+    const float room = fmaxf(vmax - (wx * ex + wy * ey) * inv, 0.0f);
     const float m = fmaxf(fminf(rintf(__fdividef(room - dv, amax * dt)), k), 0.0f);
     const float way = kd * vmax;
     const float reach = 2.0f * radius + rho[j] + dp + m * dt * dv + 0.5f * amax * dt * dt * (m * (m - 1.0f)) + (k - m) * dt * room;
     const float slack = 2e-3f + 1e-4f * (reach + way) + 4.8e-7f * (float)H * (fabsf(cx) + fabsf(cy) + way);
     const float need = reach + slack;
     if (margin) // negative: by how much it is missed
-        *margin = sqrtf(sq) - need;
+        *margin = sq * inv - need;
     return sq > need * need && sq < 1e30f;
 }
 
@@ -72,12 +73,12 @@ __device__ __forceinline__ bool clearAfter(float dt, float radius, const float* 
 // While a sample by itself can still be there, the others need no test: that takes 25
 // instructions in place of up to 100.
 // wait: after a test that failed, how many steps it takes until the reach to the witness is shorter
-// by what was missing (each takes amax dt^2 k off it), 0 where no number was missing. Tests before
-// that seldom succeed; fewer or more steps are worse. Gate race (B200, 1965 MHz), a test every
-// fourth step / waiting for all of it / half / 1.4 times / twice: control step of four agents in the
-// benchmark's state, where nothing clears, 1.006 / 0.964 / 0.970 / 0.966 / 0.990 ms (0.959 without
-// tests or tables), in three drawn mid-race states 624 584 523 / 617 577 513 / 622 579 515 /
-// 635 593 513 / 710 641 533 us.
+// by what was missing (each takes amax dt^2 k off it); 0 for 64 and more, since an infinite reach (a
+// branch that leaves the track) ends with that branch's step. Tests before that seldom succeed. Gate
+// race (B200, 1965 MHz), a test every fourth step / with the wait: control step of four agents in the
+// benchmark's state, where nothing clears, 1.008 / 0.962 ms (0.958 without tests or tables), in three
+// drawn mid-race states 627 588 525 / 616 574 513 us. Half the wait / 1.4 times / twice, against 0.964 ms
+// and 617 577 513 us of a first form: 0.970 / 0.966 / 0.990, 622 579 515 / 635 593 513 / 710 641 533.
 __device__ __forceinline__ bool clearOfEgo(float dt, float radius, const float* xy, const float* rho, int H, int t, bool active, float px, float py,
                                            float vx, float vy, float vmax, float amax, int& witness, int* wait = nullptr)
 {
@@ -115,7 +116,7 @@ __device__ __forceinline__ bool clearOfEgo(float dt, float radius, const float* 
             if (wait)
             {
                 const float miss = -__shfl_sync(ALL, margin, last);
-                *wait = miss < 1e30f ? (int)fminf(__fdividef(miss, amax * dt * dt * (float)(witness - t + 1)), (float)H) : 0;
+                *wait = (int)fminf(__fdividef(miss, amax * dt * dt * (float)(witness - t + 1)), 64.0f) & 63;
             }
             return false;
         }
